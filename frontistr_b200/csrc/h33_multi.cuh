@@ -199,10 +199,6 @@ __global__ void __launch_bounds__(kThreads) mr_spmv_kernel(SellView<double> A, c
 // cp.async.bulk on an mbarrier; the half-warps then read p from shared memory.  Each
 // p row crosses L2 once per tile instead of once per block that uses it.
 
-__device__ __forceinline__ uint32_t smem_addr(const void *p) {
-  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-
 // Waits for the mbarrier phase `parity`; bounded by two seconds of the global
 // timer (try_wait itself suspends for a bounded time), returns false when it ran out.
 __device__ __forceinline__ bool mbar_wait(uint64_t *mbar, uint32_t parity) {

@@ -1,0 +1,530 @@
+// h33_persist.cuh -- the whole CG + SSOR solve in one persistent launch.
+//
+// One iteration of hecmw_solve_CG with the SSOR preconditioner reads every block of A
+// twice when it is written as z = M^-1 r followed by q = A p: once in the sweeps, once in
+// the product.  With M = (D + L) D^-1 (D + U) built from A's own blocks (SIGMA_DIAG = 1)
+// the product needs no second reading: the forward sweep leaves g = D y with
+// (D + L) y = r, the backward sweep solves (D + U) z = g, so
+//     A z = (D + U) z + L z = g + L z,
+// and L z is one more pair of operands for the blocks that the NEXT forward sweep reads
+// anyway.  That sweep in turn need not start from the new residual: y is linear in r, so
+// it runs on the direction, (D + L) t = q, and g follows from g -= ALPHA D t as r follows
+// from r -= ALPHA q.  With v = U z from the backward sweep (D + L) u = v gives
+//     D t = h:  h = (g - L u) + BETA h_old,   q = (g + L z) + BETA q_old,
+// so the order of an iteration is
+//     backward:  v = U z,  z = D^-1 (g - v),            RHO = r.z
+//     forward:   u = D^-1 (v - L u),  p, q, h as above,  C1 = p.q
+//     update:    x += ALPHA p,  r -= ALPHA q,  g -= ALPHA h,  r.r
+// The iterates are hecmw_solve_CG's in exact arithmetic (the same RHO, C1, ALPHA, BETA
+// and tests on them); every true-residual refresh recomputes g from the new r by a plain
+// forward sweep.
+//
+// What bounds it: the colours are a chain of 2 x NColor dependent steps.  As one launch
+// per colour a step cost 5 to 10 us whatever its size (launch, ramp, tail); here one CTA
+// per SM stays for the whole solve and a grid barrier (1.1 us bare, 1.6 us with the
+// stores before it and the first load after it) separates the colours.  A small system
+// runs as one cluster of 16 CTAs, whose hardware barrier takes 0.25 us.  What is left of
+// a step is the latency of one slice per warp: a round of loads, 9 or 18 fused
+// multiply-adds per block, the lane sums, the 3x3 solve.  Measured per iteration against
+// the colour launches (us): 378 nodes 63 / 181, 19 thousand 107 / 305, 118 thousand
+// 173 / 372, 275 thousand 277 / 501, 1.03 million 705 / 1125.
+// Measured and dropped: the blocks through shared-memory rings filled by bulk copies
+// (819 to 1000 us at 1.03 million nodes: 750 instructions a slice against 300, and a
+// ring of 12 KB a warp holds little more than the slice in work); the next slice's
+// blocks held in registers (spills); bulk prefetch of the next slice into L2 (821 us);
+// 24 warps per CTA (80 registers, spills: 1129 us).
+#pragma once
+
+#include "h33_kernels.cuh"
+
+namespace h33 {
+
+// Warps per CTA, one CTA per SM.  With few rows a colour (K >= 8) 12 warps, whose 168
+// registers hold a slice without spills (107 against 111 us an iteration at 19 thousand
+// nodes); where every warp has several slices (K = 4) 16 of them (705 against 738 us at
+// 1.03 million).
+template <int K>
+constexpr int persist_warps() {
+  return K >= 8 ? 12 : 16;
+}
+constexpr int kPEnd = 0x7fffffff;            // end of a warp's list
+constexpr int kPSpin = 1 << 23;              // polls of a grid barrier before it gives up (seconds)
+
+// One sweep direction: the blocks and, for each warp of the grid, its slices in the
+// order of the sweep: (first slot, slots, first row, step << 6 | rows), kPEnd in w ends it.
+struct PersistSweep {
+  const double *val;
+  const int *col;
+  const int4 *items;
+  int stride;
+};
+
+struct PersistArgs {
+  PersistSweep lo, up;
+  SellView<double> A;
+  const double *alu;        // diagonal LU, entry e of position i at alu[e * n + i]
+  const int *perm, *iperm;  // position -> node and back
+  const double *b;          // node order
+  double *x, *r;            // node order: x in and out, r out
+  double *px, *pr, *pg, *pp, *pq, *ph;  // position order
+  double2 *zu;              // per position z and v (backward sweep) or u (forward): 3 double2
+  CgState *st;
+  const CgParams *prm;
+  double *parts;            // 3 x gridDim.x partial sums
+  unsigned *bar;            // [0] arrivals at the grid barrier, [1] set when a wait gave up
+  int n, ncolor;
+};
+
+// The slices of every warp's list: slice t of a group goes to warp t mod nw of the grid.
+static __global__ void persist_items_kernel(const int *__restrict__ gs, int ng, int reverse,
+                                            const int *__restrict__ row0, const int *__restrict__ nrows,
+                                            const int *__restrict__ slot0, const int *__restrict__ len, int nw,
+                                            int stride, int4 *__restrict__ items) {
+  const int w = blockIdx.x * blockDim.x + threadIdx.x;
+  if (w >= nw) return;
+  int4 *out = items + size_t(w) * stride;
+  int k = 0;
+  for (int c = 0; c < ng; c++) {
+    const int g = reverse ? ng - 1 - c : c;
+    for (int s = gs[g] + w; s < gs[g + 1]; s += nw) out[k++] = make_int4(slot0[s], len[s], row0[s], (c << 6) | nrows[s]);
+  }
+  for (; k < stride; k++) out[k] = make_int4(0, 0, 0, kPEnd);
+}
+
+static __global__ void invert_perm_kernel(const int *__restrict__ perm, int n, int *__restrict__ iperm) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) iperm[perm[i]] = i;
+}
+
+// ---- barriers and sums over the grid (or the cluster) ------------------------------
+struct PersistShared {
+  CgState st;
+  double red[32];
+  double val;
+  int dead;
+};
+
+// Every write made before persist_arrive by any CTA is visible after persist_wait.
+// CLUSTER: the grid is one cluster and the barrier its hardware barrier; else a counter
+// in global memory, its wait bounded.
+template <bool CLUSTER>
+__device__ __forceinline__ void persist_arrive(const PersistArgs &a, unsigned &target) {
+  if constexpr (CLUSTER) {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  } else {
+    target += gridDim.x;
+    __syncthreads();
+    if (threadIdx.x == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.bar) : "memory");
+  }
+}
+template <bool CLUSTER>
+__device__ __forceinline__ void persist_wait(const PersistArgs &a, PersistShared &sh, unsigned target) {
+  if constexpr (CLUSTER) {
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  } else {
+    if (threadIdx.x == 0) {
+      unsigned v;
+      int tries = 0;
+      for (;;) {
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(a.bar) : "memory");
+        if (int(v - target) >= 0) break;
+        if (sh.dead || ++tries > kPSpin || ((tries & 1023) == 0 && *((volatile unsigned *)(a.bar + 1)))) {
+          sh.dead = 1;
+          *((volatile unsigned *)(a.bar + 1)) = 1u;
+          break;
+        }
+      }
+    }
+    __syncthreads();
+  }
+}
+template <bool CLUSTER>
+__device__ __forceinline__ void persist_barrier(const PersistArgs &a, PersistShared &sh, unsigned &target) {
+  persist_arrive<CLUSTER>(a, target);
+  persist_wait<CLUSTER>(a, sh, target);
+}
+
+// Sum over the grid, the same value in every thread; includes a barrier.
+template <bool CLUSTER>
+__device__ __forceinline__ double persist_sum(const PersistArgs &a, PersistShared &sh, unsigned &target, double v,
+                                              int slot) {
+  v = block_sum(v, sh.red);
+  double *parts = a.parts + slot * gridDim.x;
+  if (threadIdx.x == 0) parts[blockIdx.x] = v;
+  persist_barrier<CLUSTER>(a, sh, target);
+  if (threadIdx.x < 32) {
+    double s = 0.0;
+    for (int i = threadIdx.x; i < int(gridDim.x); i += 32) s += __ldcg(parts + i);
+    s = warp_sum(s);
+    if (threadIdx.x == 0) sh.val = s;
+  }
+  __syncthreads();
+  return sh.val;
+}
+
+// ---- one slice ----------------------------------------------------------------------
+// Loads of what other CTAs wrote: coherent after a barrier, never the read-only path.
+template <bool L2ONLY, class T>
+__device__ __forceinline__ T ld_row(const T *p) {
+  if constexpr (L2ONLY) return __ldcg(p);
+  else return *p;
+}
+
+// One sweep, MODE 0 backward, 1 forward on the direction, 2 forward from r (start and
+// refresh): the colours in turn, a barrier between them.  K lanes per row; lane c < 3 of
+// a row (MODE 1, K >= 8: of each half of its lanes) carries component c of its vectors.
+// The columns of the slice whose turn is next are loaded before the barrier, so that
+// what follows it is one round of loads: blocks, diagonal LU, own vectors, gathers.
+template <int K, int MODE, bool CLUSTER>
+__device__ __forceinline__ double persist_sweep(const PersistArgs &a, PersistShared &sh, unsigned &target, int w,
+                                                double beta, bool first) {
+  constexpr int U = 2;                          // slots taken together (4: more registers, no faster)
+  constexpr bool HALVES = MODE == 1 && K >= 8;  // a row's upper lanes end with the sums over z, the lower over u
+  const int lane = threadIdx.x & 31;
+  const int sub = lane & (K - 1), roff = lane / K;
+  const bool up = HALVES && (sub & (K / 2)) != 0;
+  const int cc = HALVES ? sub & (K / 2 - 1) : sub, c0 = min(cc, 2);
+  const PersistSweep S = MODE == 0 ? a.up : a.lo;
+  const int4 *items = S.items + size_t(w) * S.stride;
+  const size_t n = size_t(a.n);
+  double dot = 0.0;
+  int4 it = __ldg(items), nx = __ldg(items + 1);
+  items += 2;
+  int col[U];
+#pragma unroll
+  for (int u = 0; u < U; u++) col[u] = u < it.y ? __ldg(S.col + (it.x + u) * 32 + lane) : 0;
+  for (int c = 0; c < a.ncolor; c++) {
+    if (c) persist_barrier<CLUSTER>(a, sh, target);
+    while ((it.w >> 6) == c) {
+      const bool act = roff < (it.w & 63);
+      const int row = it.z + (act ? roff : 0), i3 = 3 * row;
+      const double *lu = a.alu + row;
+      const double a0 = __ldcs(lu), a1 = __ldcs(lu + n), a2 = __ldcs(lu + 2 * n);
+      const double a3 = __ldcs(lu + 3 * n), a4 = __ldcs(lu + 4 * n), a5 = __ldcs(lu + 5 * n);
+      const double a6 = __ldcs(lu + 6 * n), a7 = __ldcs(lu + 7 * n), a8 = __ldcs(lu + 8 * n);
+      double o0, o1, o2;  // the row's own right-hand side: g, v or r
+      double f0 = 0.0, f1 = 0.0, f2 = 0.0, f3 = 0.0, f4 = 0.0;
+      const double *own = reinterpret_cast<const double *>(a.zu + 3 * size_t(row));
+      if (MODE == 1) {
+        o0 = __ldcg(own + 3), o1 = __ldcg(own + 4), o2 = __ldcg(own + 5);
+        f0 = __ldcg(a.pg + i3 + c0);
+        if (HALVES) {
+          if (!first) f1 = __ldcg((up ? a.pq : a.ph) + i3 + c0);
+          if (up) {
+            f2 = __ldcg(own + c0);
+            if (!first) f3 = __ldcg(a.pp + i3 + c0);
+          }
+        } else {
+          f2 = __ldcg(own + c0);
+          if (!first) {
+            f1 = __ldcg(a.ph + i3 + c0);
+            f3 = __ldcg(a.pp + i3 + c0);
+            f4 = __ldcg(a.pq + i3 + c0);
+          }
+        }
+      } else {
+        const double *src = (MODE == 0 ? a.pg : a.pr) + i3;
+        o0 = __ldcg(src), o1 = __ldcg(src + 1), o2 = __ldcg(src + 2);
+        if (MODE == 0) f0 = __ldcg(a.pr + i3 + c0);
+      }
+      double l[3] = {0.0, 0.0, 0.0}, m[3] = {0.0, 0.0, 0.0};  // sums over u (z when MODE 0), and over z
+      for (int s = 0; s < it.y; s += U) {
+        const int nu = it.y - s;
+        double2 ga[U], gb[U], gd[U];
+        double v[U][9];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+          ga[u] = gb[u] = gd[u] = make_double2(0.0, 0.0);
+#pragma unroll
+          for (int e = 0; e < 9; e++) v[u][e] = 0.0;
+          if (u < nu) {
+            const double2 *g = a.zu + 3 * size_t(col[u]);
+            if (MODE != 2) ga[u] = ld_row<CLUSTER>(g);
+            gb[u] = ld_row<CLUSTER>(g + 1);
+            if (MODE != 0) gd[u] = ld_row<CLUSTER>(g + 2);
+            const double *b = S.val + size_t(it.x + s + u) * 288 + lane;
+#pragma unroll
+            for (int e = 0; e < 9; e++) v[u][e] = __ldcs(b + 32 * e);
+          }
+        }
+        // the columns after these: the slice's next slots, or the next slice's first
+        const bool more = nu > U;
+        const int slot = more ? it.x + s + U : nx.x, left = more ? nu - U : nx.y;
+#pragma unroll
+        for (int u = 0; u < U; u++)
+          if (u < left) col[u] = __ldg(S.col + (slot + u) * 32 + lane);
+#pragma unroll
+        for (int u = 0; u < U; u++)
+          if (u < nu) {
+#pragma unroll
+            for (int i = 0; i < 3; i++) {
+              const double v0 = v[u][3 * i], v1 = v[u][3 * i + 1], v2 = v[u][3 * i + 2];
+              if (MODE == 0) l[i] = fma(v2, gb[u].x, fma(v1, ga[u].y, fma(v0, ga[u].x, l[i])));
+              else l[i] = fma(v2, gd[u].y, fma(v1, gd[u].x, fma(v0, gb[u].y, l[i])));
+              if (MODE == 1) m[i] = fma(v2, gb[u].x, fma(v1, ga[u].y, fma(v0, ga[u].x, m[i])));
+            }
+          }
+      }
+      if (it.y == 0) {
+#pragma unroll
+        for (int u = 0; u < U; u++)
+          if (u < nx.y) col[u] = __ldg(S.col + (nx.x + u) * 32 + lane);
+      }
+      if (HALVES) {
+#pragma unroll
+        for (int j = 0; j < 3; j++) {
+          const double other = __shfl_xor_sync(0xffffffffu, up ? l[j] : m[j], K / 2);
+          l[j] = (up ? m[j] : l[j]) + other;
+        }
+      }
+#pragma unroll
+      for (int o = HALVES ? K / 4 : K / 2; o > 0; o >>= 1) {
+#pragma unroll
+        for (int j = 0; j < 3; j++) {
+          l[j] += __shfl_xor_sync(0xffffffffu, l[j], o);
+          if (MODE == 1 && !HALVES) m[j] += __shfl_xor_sync(0xffffffffu, m[j], o);
+        }
+      }
+      const double e0 = o0 - l[0], e1 = o1 - l[1], e2 = o2 - l[2];
+      double x1 = e0, x2 = e1, x3 = e2;  // D^-1 e by the reciprocal-pivot LU
+      x2 = x2 - a3 * x1;
+      x3 = x3 - a6 * x1 - a7 * x2;
+      x3 = a8 * x3;
+      x2 = a4 * (x2 - a5 * x3);
+      x1 = a0 * (x1 - a2 * x3 - a1 * x2);
+      if (act && cc < 3) {
+        const int i = i3 + cc;
+        const double xc = cc == 0 ? x1 : cc == 1 ? x2 : x3;
+        const double lc = cc == 0 ? l[0] : cc == 1 ? l[1] : l[2];
+        double *uo = reinterpret_cast<double *>(a.zu + 3 * size_t(row)) + 3 + cc;
+        if (MODE == 0) {  // z = D^-1 (g - U z) and v = U z
+          a.zu[3 * size_t(row) + cc] =
+              cc == 0 ? make_double2(x1, x2) : cc == 1 ? make_double2(x3, l[0]) : make_double2(l[1], l[2]);
+          dot += f0 * xc;
+        } else if (MODE == 2) {
+          *uo = xc;
+          a.pg[i] = cc == 0 ? e0 : cc == 1 ? e1 : e2;
+        } else if (HALVES) {
+          const double t = up ? f0 + lc : f0 - lc;  // g + L z, or g - L u
+          const double tn = first ? t : t + beta * f1;
+          (up ? a.pq : a.ph)[i] = tn;
+          if (up) {
+            const double pn = first ? f2 : f2 + beta * f3;
+            a.pp[i] = pn;
+            dot += pn * tn;
+          } else {
+            *uo = xc;
+          }
+        } else {
+          const double mc = cc == 0 ? m[0] : cc == 1 ? m[1] : m[2];
+          double pn = f2, qn = f0 + mc, hn = f0 - lc;
+          if (!first) {
+            pn = pn + beta * f3;
+            qn = qn + beta * f4;
+            hn = hn + beta * f1;
+          }
+          *uo = xc;
+          a.pp[i] = pn;
+          a.pq[i] = qn;
+          a.ph[i] = hn;
+          dot += pn * qn;
+        }
+      }
+      it = nx;
+      nx = __ldg(items);
+      if (nx.w != kPEnd) items++;
+    }
+  }
+  return dot;
+}
+
+// r = b - A x from x in node order, r in position order; |r|^2 or (BB) |b|^2.
+template <bool BB>
+__device__ __forceinline__ double persist_resid(const PersistArgs &a) {
+  const int lane = threadIdx.x & 31;
+  const int nw = (gridDim.x * blockDim.x) >> 5;
+  double acc = 0.0;
+  for (int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; s < a.A.nslices; s += nw) {
+    const bool active = lane < a.A.nrows[s];
+    const int row = a.A.row0[s] + lane;
+    const int len = active ? a.A.rowlen[s * 32 + lane] : 0;
+    double y0 = 0.0, y1 = 0.0, y2 = 0.0;
+    row_gemv<double, double, 1, false, true>(a.A, s, lane, len, a.x, y0, y1, y2);
+    if (active) {
+      const double b0 = a.b[3 * row], b1 = a.b[3 * row + 1], b2 = a.b[3 * row + 2];
+      y0 = b0 - y0;
+      y1 = b1 - y1;
+      y2 = b2 - y2;
+      const int i3 = 3 * a.iperm[row];
+      a.pr[i3] = y0;
+      a.pr[i3 + 1] = y1;
+      a.pr[i3 + 2] = y2;
+      acc += BB ? b0 * b0 + b1 * b1 + b2 * b2 : y0 * y0 + y1 * y1 + y2 * y2;
+    }
+  }
+  return acc;
+}
+
+template <int K, bool CLUSTER>
+__global__ void __launch_bounds__(32 * persist_warps<K>(), 1) cg_ssor_persist_kernel(const PersistArgs a) {
+  __shared__ PersistShared sh;
+  const int tid = threadIdx.x, warp = tid >> 5;
+  const int w = warp * gridDim.x + blockIdx.x;  // this warp's list: neighbouring slices on different SMs
+  const int gt = blockIdx.x * blockDim.x + tid, nt = gridDim.x * blockDim.x;
+  unsigned target = 0;
+  if (tid == 0) {
+    CgState &st = sh.st;
+    st.rho = st.rho1 = st.alpha = st.beta = st.pq = st.rr = 0.0;
+    st.bnrm2 = st.resid = st.rr_true = 0.0;
+    st.tol = a.prm->tol;
+    st.maxit = a.prm->maxit;
+    st.iter = 1;
+    st.done = st.error = st.n_indef = st.recompute = st.converged = st.zero_rhs = 0;
+    st.guard = 0;
+    st.inner = st.flexible = st.use_gnn = st.restart = st.fallback = 0;
+    st.omega = st.c2 = 0.0;
+    st.nrecompute = kIterRecomputeR;
+    st.resid_mark = 1.0;
+    st.gamma = 1.0f;
+    st.reliable = st.ru_pending = st.ru_count = 0;
+    st.ru_delta = a.prm->ru_delta;
+    st.ru_mark = 1.0;
+    const bool log = blockIdx.x == 0;  // every CTA takes the same decisions, one records them
+    st.lanczos = log ? a.prm->lanczos : nullptr;
+    st.lanczos_cap = a.prm->lanczos_cap;
+    st.rhist = log ? a.prm->rhist : nullptr;
+    st.rhist_cap = a.prm->rhist_cap;
+    st.lanczos_n = st.rhist_n = 0;
+    for (int i = 0; i < 8; i++) st.ticket[i] = 0u;
+    sh.dead = 0;
+  }
+  __syncthreads();
+  // x in position order; z and u start at zero (padding blocks gather position 0)
+  for (int i = gt; i < a.n; i += nt) {
+    const int node = a.perm[i];
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      a.px[3 * i + c] = a.x[3 * node + c];
+      a.zu[3 * size_t(i) + c] = make_double2(0.0, 0.0);
+    }
+  }
+  CgState &st = sh.st;
+  {
+    const double bb = persist_sum<CLUSTER>(a, sh, target, persist_resid<true>(a), 0);
+    if (tid == 0) {
+      st.bnrm2 = bb;
+      if (bb == 0.0) {
+        st.zero_rhs = 1;
+        st.done = 1;
+      }
+      if (st.maxit <= 0) st.done = 1;
+    }
+    __syncthreads();
+  }
+  const int n3 = 3 * a.n, n2 = n3 / 2;
+  bool restart = true;  // g from r
+  while (!st.done) {
+    if (restart) {
+      persist_sweep<K, 2, CLUSTER>(a, sh, target, w, 0.0, false);
+      persist_barrier<CLUSTER>(a, sh, target);
+      restart = false;
+    }
+    if (tid == 0) st.guard++;
+    const double rho = persist_sum<CLUSTER>(a, sh, target, persist_sweep<K, 0, CLUSTER>(a, sh, target, w, 0.0, false), 0);
+    if (tid == 0) fin_rho(&st, rho);
+    __syncthreads();
+    if (st.done) break;
+    const bool first = st.iter == 1;
+    const double pq =
+        persist_sum<CLUSTER>(a, sh, target, persist_sweep<K, 1, CLUSTER>(a, sh, target, w, st.beta, first), 1);
+    if (tid == 0) fin_pq(&st, pq);
+    __syncthreads();
+    if (st.done) break;
+    const bool refresh = (st.iter % st.nrecompute) == 0;
+    {
+      const double alpha = st.alpha;
+      double rr = 0.0;
+      double2 *x2 = reinterpret_cast<double2 *>(a.px), *r2 = reinterpret_cast<double2 *>(a.pr),
+              *g2 = reinterpret_cast<double2 *>(a.pg);
+      const double2 *p2 = reinterpret_cast<const double2 *>(a.pp), *q2 = reinterpret_cast<const double2 *>(a.pq),
+                    *h2 = reinterpret_cast<const double2 *>(a.ph);
+      for (int i = gt; i < n2; i += nt) {
+        double2 x = __ldcg(x2 + i);
+        const double2 p = __ldcg(p2 + i);
+        x.x = alpha * p.x + x.x;
+        x.y = alpha * p.y + x.y;
+        x2[i] = x;
+        if (!refresh) {
+          double2 r = __ldcg(r2 + i), g = __ldcg(g2 + i);
+          const double2 q = __ldcg(q2 + i), h = __ldcg(h2 + i);
+          r.x = -alpha * q.x + r.x;
+          r.y = -alpha * q.y + r.y;
+          g.x = -alpha * h.x + g.x;
+          g.y = -alpha * h.y + g.y;
+          r2[i] = r;
+          g2[i] = g;
+          rr += r.x * r.x + r.y * r.y;
+        }
+      }
+      if (gt == nt - 1 && (n3 & 1)) {
+        const int i = n3 - 1;
+        a.px[i] = alpha * __ldcg(a.pp + i) + __ldcg(a.px + i);
+        if (!refresh) {
+          const double r = -alpha * __ldcg(a.pq + i) + __ldcg(a.pr + i);
+          a.pr[i] = r;
+          a.pg[i] = -alpha * __ldcg(a.ph + i) + __ldcg(a.pg + i);
+          rr += r * r;
+        }
+      }
+      if (refresh) persist_barrier<CLUSTER>(a, sh, target);
+      else {
+        rr = persist_sum<CLUSTER>(a, sh, target, rr, 2);
+        if (tid == 0) fin_rr(&st, rr);
+        __syncthreads();
+      }
+    }
+    if (refresh || st.recompute) {
+      for (int i = gt; i < a.n; i += nt) {
+        const int node = a.perm[i];
+#pragma unroll
+        for (int c = 0; c < 3; c++) a.x[3 * node + c] = __ldcg(a.px + 3 * i + c);
+      }
+      persist_barrier<CLUSTER>(a, sh, target);
+      const double rr = persist_sum<CLUSTER>(a, sh, target, persist_resid<false>(a), 2);
+      if (tid == 0) {
+        st.rr = rr;
+        st.resid = sqrt(rr / st.bnrm2);
+        if (refresh) record_resid(&st);
+        if (st.resid <= st.tol) {
+          st.done = 1;
+          st.converged = 1;
+        }
+      }
+      restart = true;
+    }
+    if (tid == 0) {
+      loop_ctl(&st, 0, 0);
+      if (sh.dead) st.done = 1;
+    }
+    __syncthreads();
+  }
+  if (!sh.dead && !st.zero_rhs) {
+    for (int i = gt; i < a.n; i += nt) {
+      const int node = a.perm[i];
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+        a.x[3 * node + c] = __ldcg(a.px + 3 * i + c);
+        a.r[3 * node + c] = __ldcg(a.pr + 3 * i + c);
+      }
+    }
+  }
+  if (blockIdx.x == 0 && tid == 0) {
+    if (sh.dead) {
+      st.error = HECMW33_ERR_TIMEOUT;
+      st.done = 1;
+    }
+    *a.st = st;
+  }
+  if constexpr (CLUSTER) persist_barrier<true>(a, sh, target);
+}
+
+}  // namespace h33

@@ -41,6 +41,7 @@
 #include "h33_kernels.cuh"
 #include "h33_layout.cuh"
 #include "h33_multi.cuh"
+#include "h33_persist.cuh"
 #include "h33_setup.h"
 #include "h33_vecops.cuh"
 
@@ -170,6 +171,18 @@ int sweep_lanes() {
   return (k == 4 || k == 8 || k == 16) ? k : 4;
 }
 
+// The same for the SSOR of a CG solve, whose rows per colour (n / ncolor) decide: the more
+// lanes a row has the shorter a step of cg_ssor_persist_kernel, until its slices are
+// about half as many as the grid's warps (12 a CTA).  Measured per iteration with
+// 4 / 8 / 16 lanes (us): 1,105 rows a colour 133 / 115 / 108, 3,135 rows 146 / 126 / 145,
+// 7,350 rows 171 / 182 / 235, 17 thousand 272 / 317.
+int ssor_lanes(int n, int ncolor, int nsm) {
+  if (std::getenv("HECMW33_SWEEP_LANES")) return sweep_lanes();
+  const int64_t rows = n / std::max(ncolor, 1);
+  if (rows <= 12 * nsm) return 16;
+  return rows <= 24 * nsm ? 8 : 4;
+}
+
 double wall() {
   return std::chrono::duration<double>(std::chrono::steady_clock::now().time_since_epoch()).count();
 }
@@ -270,6 +283,18 @@ struct Precond {
   int numeric_version = 0, fp32_version = -1, lowp_version = -1;
   bool pos_cols = false;  // lo/up columns are colour positions (multicolour SSOR)
   double sigma = 0.0;     // SIGMA_DIAG of the last numeric setup
+  int values_version = -1;  // matrix values (Solver::values_version) of the last numeric setup
+};
+
+// The persistent CG's per-warp slice lists and workspace for one SSOR layout.
+struct PersistPlan {
+  int generation = -1;   // Precond::generation it was made for
+  int grid = 0, lo_stride = 0, up_stride = 0;
+  bool cluster = false;
+  DevArray<int4> lo_items, up_items;
+  DevArray<int> iperm;
+  DevArray<double> zu, parts;
+  DevArray<unsigned> bar;
 };
 
 // The learned preconditioner: node graph of the matrix, weights, activations and
@@ -415,6 +440,7 @@ struct Solver {
   CgState *h_state = nullptr;
   DevArray<int> d_err;
   Precond pc;
+  PersistPlan pp;
   // FP32 copies for the mixed-precision refinement
   DevArray<float> bf, xf, rf, zf, pf, qf, wf, zpf;
   // flexible CG buffers (SSOR output and previous residual) and the learned preconditioner
@@ -891,7 +917,9 @@ void diag_alu(Solver &S, DevArray<double> &alu, const double *blocks, const int 
 // SSOR in P: the reference's RCM + multicolour ordering (greedy = false, the drop-in),
 // or first-fit colours in the input order (greedy = true: the learned preconditioner's
 // smoother, which is not bound to the reference's schedule).
-void setup_ssor(Solver &S, Precond &P, int ncolor_in, double sigma, bool symbolic, bool greedy) {
+// cg: the lanes per row are the persistent CG's; the other methods and the smoother keep
+// sweep_lanes() for the launches per colour.
+void setup_ssor(Solver &S, Precond &P, int ncolor_in, double sigma, bool symbolic, bool greedy, bool cg) {
   P.sigma = sigma;
   if (symbolic) {
     Profile prof{S.N, S.indexL.data(), S.itemL.data(), S.indexU.data(), S.itemU.data()};
@@ -906,7 +934,7 @@ void setup_ssor(Solver &S, Precond &P, int ncolor_in, double sigma, bool symboli
       P.ncolor = ordering_mc(prof, perm_rcm, ncolor_in, colorindex, perm, iperm);
       setup_mark("ssor: multicolouring");
     }
-    const int lanes = sweep_lanes();
+    const int lanes = cg ? ssor_lanes(S.N, P.ncolor, S.nsm) : sweep_lanes();
     if (host_layouts()) {
       BlockRows lower_ref, upper_ref, lower, upper;
       reordered_rows(prof, perm, iperm, lower_ref, upper_ref);
@@ -1004,6 +1032,7 @@ void setup_ssor(Solver &S, Precond &P, int ncolor_in, double sigma, bool symboli
   P.lo.pack(S.raw.p, S.stream, S.nsm);
   P.up.pack(S.raw.p, S.stream, S.nsm);
   diag_alu(S, P.alu_fwd, S.raw.p, P.perm_fwd.p, sigma, 0);
+  P.values_version = S.values_version;
   setup_mark("ssor: value packing + diagonal LU");
 }
 
@@ -1163,7 +1192,7 @@ void precond_setup(Solver &S, int precond, int ncolor_in, double sigma, int *Iar
   }
   P.kind = kind;
   P.ncolor_in = ncolor_in;
-  if (kind == 1) setup_ssor(S, P, ncolor_in, sigma, symbolic, false);
+  if (kind == 1) setup_ssor(S, P, ncolor_in, sigma, symbolic, false, Iarray[1] == 1);
   else if (kind == 3) diag_alu(S, P.alu_fwd, S.raw.p, nullptr, sigma, 0);
   else setup_bilu(S, level, sigma, symbolic);
   int err = 0;
@@ -1191,7 +1220,7 @@ void ensure_smoother(Solver &S) {
   if (!symbolic && L.sm_numeric_for == S.pc.numeric_version) return;
   if (symbolic) P = Precond();
   P.kind = 1;
-  setup_ssor(S, P, 0, S.pc.sigma, symbolic, true);
+  setup_ssor(S, P, 0, S.pc.sigma, symbolic, true, false);
   int err = 0;
   H33_CUDA(cudaMemcpyAsync(&err, S.d_err.p, sizeof(int), cudaMemcpyDeviceToHost, S.stream));
   S.sync();
@@ -1772,6 +1801,170 @@ float run_cg(Solver &S, int iterpremax, double tol, int maxit, int *kernels, int
   const CgState &st = *S.h_state;
   if (!st.done && !st.zero_rhs)
     throw Failure(HECMW33_ERR_TIMEOUT, "device CG loop ended without a decision (internal error)");
+  return ms;
+}
+
+// Whether the plain FP64 CG of this solve can run as cg_ssor_persist_kernel: SSOR in the
+// colour layout with SIGMA_DIAG = 1, built from the very values of the resident matrix
+// (a recycled preconditioner is not A's own triangles any more).
+bool persist_ok(const Solver &S, int iterpremax) {
+  const Precond &P = S.pc;
+  return P.valid && P.kind == 1 && P.pos_cols && iterpremax == 1 && P.sigma == 1.0 &&
+         P.values_version == S.values_version;
+}
+
+template <int K, bool CLUSTER>
+void persist_config(Solver &S, int grid, cudaLaunchConfig_t &cfg, cudaLaunchAttribute *attr) {
+  cfg = {};
+  cfg.gridDim = dim3(unsigned(grid), 1, 1);
+  cfg.blockDim = dim3(32 * persist_warps<K>(), 1, 1);
+  cfg.stream = S.stream;
+  if (CLUSTER) {
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = unsigned(grid);
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  } else {
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+  }
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+}
+
+// CTAs of the launch, negative for one cluster of that many: a cluster of 16 (of 8 where
+// the device cannot place 16) while a colour's rows fit its warps at 16 lanes a row once
+// (384 rows; 69 us an iteration against 89 us on the whole grid at 143 rows a colour),
+// else a CTA per SM.
+template <int K>
+int persist_grid(Solver &S, int rows) {
+  constexpr int W = persist_warps<K>();
+  if constexpr (K == 16) {
+    auto kern = cg_ssor_persist_kernel<K, true>;
+    H33_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    for (int c : {16, 8}) {
+      if (rows > 2 * c * W) break;
+      cudaLaunchConfig_t cfg;
+      cudaLaunchAttribute attr[1];
+      persist_config<K, true>(S, c, cfg, attr);
+      int n = 0;
+      if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess && n > 0) return -c;
+      cudaGetLastError();
+    }
+  }
+  int per_sm = 0;
+  H33_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cg_ssor_persist_kernel<K, false>, 32 * W, 0));
+  if (per_sm < 1) throw Failure(HECMW33_ERR_CUDA, "the persistent CG does not fit an SM");
+  return S.nsm;
+}
+
+template <int K>
+void persist_plan(Solver &S) {
+  PersistPlan &L = S.pp;
+  const Precond &P = S.pc;
+  if (L.generation == P.generation) return;
+  const int ng = int(P.lo.group_slice.size()) - 1;
+  const int grid = persist_grid<K>(S, S.N / std::max(ng, 1));
+  L.cluster = grid < 0;
+  L.grid = std::abs(grid);
+  const int nw = L.grid * persist_warps<K>();
+  auto lists = [&](const DevSell<double> &D, bool reverse, DevArray<int4> &items, int &stride) {
+    stride = 2;
+    for (int g = 0; g < ng; g++) stride += (D.group_slice[size_t(g) + 1] - D.group_slice[size_t(g)] + nw - 1) / nw;
+    DevArray<int> gs;
+    gs.upload(D.group_slice, S.stream);
+    items.alloc(size_t(nw) * size_t(stride));
+    launch_k(S.stream, persist_items_kernel, (nw + 63) / 64, 64, static_cast<const int *>(gs.p), ng, reverse ? 1 : 0,
+             static_cast<const int *>(D.row0.p), static_cast<const int *>(D.nrows.p),
+             static_cast<const int *>(D.slot0.p), static_cast<const int *>(D.len.p), nw, stride, items.p);
+    H33_CUDA(cudaGetLastError());
+    S.sync();
+  };
+  lists(P.lo, false, L.lo_items, L.lo_stride);
+  lists(P.up, true, L.up_items, L.up_stride);
+  L.iperm.alloc(size_t(S.N));
+  launch_k(S.stream, invert_perm_kernel, S.grid_vec(), kThreads, static_cast<const int *>(P.perm_fwd.p), S.N, L.iperm.p);
+  H33_CUDA(cudaGetLastError());
+  L.zu.alloc(6 * size_t(S.N));
+  L.parts.alloc(3 * size_t(L.grid));
+  L.bar.alloc(2);
+  L.generation = P.generation;
+}
+
+template <int K>
+void launch_persist(Solver &S, const PersistArgs &a) {
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute attr[1];
+  if constexpr (K == 16) {
+    if (S.pp.cluster) {
+      persist_config<K, true>(S, S.pp.grid, cfg, attr);
+      H33_CUDA(cudaLaunchKernelEx(&cfg, cg_ssor_persist_kernel<K, true>, a));
+      return;
+    }
+  }
+  persist_config<K, false>(S, S.pp.grid, cfg, attr);
+  H33_CUDA(cudaLaunchKernelEx(&cfg, cg_ssor_persist_kernel<K, false>, a));
+}
+
+// As run_cg for the plain FP64 CG, the whole solve in one cg_ssor_persist_kernel.
+float run_cg_persist(Solver &S, double tol, int maxit, int *kernels) {
+  const Precond &P = S.pc;
+  switch (P.lo.lanes) {
+    case 8: persist_plan<8>(S); break;
+    case 16: persist_plan<16>(S); break;
+    default: persist_plan<4>(S); break;
+  }
+  const PersistPlan &L = S.pp;
+  CgParams &h = *S.h_params;
+  h = CgParams{};
+  h.tol = tol;
+  h.maxit = maxit;
+  h.iterpremax = 1;
+  h.method = 1;
+  h.ru_delta = 1e-4;
+  h.lanczos = S.lanczos_on ? S.lanczos_buf.p : nullptr;
+  h.lanczos_cap = S.lanczos_on ? int(S.lanczos_buf.n / 2) : 0;
+  h.rhist = S.rhist_on ? S.rhist_buf.p : nullptr;
+  h.rhist_cap = S.rhist_on ? int(S.rhist_buf.n) : 0;
+  PersistArgs a;
+  a.lo = PersistSweep{P.lo.val.p, P.lo.col.p, L.lo_items.p, L.lo_stride};
+  a.up = PersistSweep{P.up.val.p, P.up.col.p, L.up_items.p, L.up_stride};
+  a.A = S.A.view();
+  a.alu = P.alu_fwd.p;
+  a.perm = P.perm_fwd.p;
+  a.iperm = L.iperm.p;
+  a.b = S.b.p;
+  a.x = S.x.p;
+  a.r = S.r.p;
+  // the solve's work vectors, here in position order
+  a.px = S.w.p;
+  a.pr = S.zp.p;
+  a.pg = S.z.p;
+  a.pp = S.p.p;
+  a.pq = S.q.p;
+  a.ph = S.zpos.p;
+  a.zu = reinterpret_cast<double2 *>(L.zu.p);
+  a.st = S.state.p;
+  a.prm = S.params.p;
+  a.parts = L.parts.p;
+  a.bar = L.bar.p;
+  a.n = S.N;
+  a.ncolor = int(P.lo.group_slice.size()) - 1;
+  H33_CUDA(cudaMemcpyAsync(S.params.p, S.h_params, sizeof(CgParams), cudaMemcpyHostToDevice, S.stream));
+  H33_CUDA(cudaMemsetAsync(S.pp.bar.p, 0, 2 * sizeof(unsigned), S.stream));
+  H33_CUDA(cudaEventRecord(S.ev0, S.stream));
+  switch (P.lo.lanes) {
+    case 8: launch_persist<8>(S, a); break;
+    case 16: launch_persist<16>(S, a); break;
+    default: launch_persist<4>(S, a); break;
+  }
+  H33_CUDA(cudaEventRecord(S.ev1, S.stream));
+  H33_CUDA(cudaMemcpyAsync(S.h_state, S.state.p, sizeof(CgState), cudaMemcpyDeviceToHost, S.stream));
+  S.sync();
+  if (kernels) *kernels += 1;
+  float ms = 0.0f;
+  H33_CUDA(cudaEventElapsedTime(&ms, S.ev0, S.ev1));
+  if (S.h_state->error == HECMW33_ERR_TIMEOUT)
+    throw Failure(HECMW33_ERR_TIMEOUT, "a wait of the persistent CG gave up (internal error)");
   return ms;
 }
 
@@ -3385,17 +3578,20 @@ int solve_fp64(Solver &S, int *Iarray, double *Rarray, int *iter, double *resid,
   S.rhist_on = Iarray[20] == 1 && (method == 1 || method == 2) && !learned;  // hecmw_mat_get_iterlog
   S.iterlog = Iarray[20] == 1;
   if (S.rhist_on) S.rhist_buf.alloc(size_t(std::max(MAXIT, 1)));
-  if (lowp && iterPREmax > 0) {
+  const bool record = S.L.recording && !learned && method == 1;
+  // the fused CG reads the FP64 blocks once per iteration, fewer bytes than BF16 sweeps
+  // and an FP64 product: precision mode 1 takes it too
+  const auto persist = [&] { return method == 1 && !learned && !record && persist_ok(S, iterPREmax); };
+  if (!lowp || iterPREmax <= 0) {
+    lowp = 0;
+  } else if (!persist()) {
     // a learned solve sweeps with its smoother only: the solve's SSOR needs its BF16
     // copy when a plain solve (or the METHOD2 hand-over below) uses it
     if (learned) ensure_lowp(S, S.L.sm);
     else ensure_lowp(S);
-  } else {
-    lowp = 0;
   }
   setup_mark("solve: BF16 copies, buffers");
-  const bool record = S.L.recording && !learned && method == 1;
-  if (graph_mode() && !record && (method == 1 || method == 2))
+  if (graph_mode() && !record && !persist() && (method == 1 || method == 2))
     build_graph<double>(S, iterPREmax, learned | (lowp ? 4 : 0) | (method == 2 ? 8 : 0));
   setup_mark("solve: graph capture + instantiate");
   Range rs("hecmw33_solve");
@@ -3416,6 +3612,7 @@ int solve_fp64(Solver &S, int *Iarray, double *Rarray, int *iter, double *resid,
                              iter, resid);
     } else {
       if (record) ms_total += record_cg(S, iterPREmax, TOL, MAXIT, &kernels);
+      else if (persist()) ms_total += run_cg_persist(S, TOL, MAXIT, &kernels);
       else ms_total += run_cg<double>(S, iterPREmax, TOL, MAXIT, &kernels, 0, learned, 0, 1e-4, lowp, method);
       const CgState &st = *S.h_state;
       error = st.error;

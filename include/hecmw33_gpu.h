@@ -45,7 +45,10 @@
  *                  = 1  mixed precision, low-precision preconditioner: FP64 CG whose
  *                       preconditioner sweeps read BF16-stored factors (FP32 diagonal
  *                       LU) and compute in FP64; matrix, vectors, dots and residuals
- *                       stay FP64, so the convergence test is the reference's
+ *                       stay FP64, so the convergence test is the reference's.  CG with
+ *                       an SSOR of the current values (one pass, SIGMA_DIAG = 1) runs as
+ *                       in mode 0: it reads each FP64 block once per iteration, fewer
+ *                       bytes than BF16 sweeps beside an FP64 product
  *                  = 2  mixed precision, restarted refinement: inner FP32 CG (FP32
  *                       matrix and preconditioner copies, FP64 dot products) from zero
  *                       to Rarray(42) relative (0 -> 1e-4), FP64 correction and true

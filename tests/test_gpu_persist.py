@@ -1,0 +1,99 @@
+"""The one-launch CG + SSOR solve (cg_ssor_persist_kernel) against the oracle, at the
+sizes where its launch shape changes: one cluster or the whole grid, 16, 8 or 4 lanes per
+row, colours with fewer rows than a slice, rows longer than what a lane takes at once."""
+import numpy as np
+import pytest
+
+from frontistr_b200.matrix import HecMatrix
+from frontistr_b200.mesh import box_system
+from frontistr_b200.solver import GpuSolver
+from oracle_ctypes import Oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def hub_system(n=220, hubs=(3, 117, 219), seed=4):
+    """A chain of n nodes with a few nodes coupled to nearly all others (rows of some 200
+    blocks), symmetric and diagonally dominant."""
+    rng = np.random.default_rng(seed)
+    pairs = {(i + 1, i) for i in range(n - 1)}
+    for h in hubs:
+        pairs |= {(max(h, j), min(h, j)) for j in range(n) if j != h and rng.random() < 0.9}
+    low = {p: rng.uniform(-1, 1, (3, 3)) for p in pairs}
+    diag = [np.eye(3) for _ in range(n)]
+    for (i, j), b in low.items():
+        w = np.abs(b).sum()
+        diag[i] = diag[i] + w * np.eye(3)
+        diag[j] = diag[j] + w * np.eye(3)
+    lows = [sorted(j for (i, j) in pairs if i == k) for k in range(n)]
+    ups = [sorted(i for (i, j) in pairs if j == k) for k in range(n)]
+    ptr = lambda rows: np.concatenate([[0], np.cumsum([len(r) for r in rows])])  # noqa: E731
+    m = HecMatrix(n, n, ptr(lows), np.concatenate(lows) + 1, ptr(ups), np.concatenate(ups) + 1,
+                  np.concatenate([d.ravel() for d in diag]),
+                  np.concatenate([low[(k, j)].ravel() for k in range(n) for j in lows[k]]),
+                  np.concatenate([low[(i, k)].T.ravel() for k in range(n) for i in ups[k]]))
+    m.B[:] = rng.standard_normal(3 * n)
+    return m
+
+
+SYSTEMS = {
+    "box_1x1x1": lambda: box_system(1, 1, 1),
+    "box_2x1x3": lambda: box_system(2, 1, 3),
+    "hubs": hub_system,
+    "cluster_14x14x20": lambda: box_system(14, 14, 20, jitter=0.2, sigma_E=1.0, nu_range=(0.25, 0.40), seed=3),
+    "grid16_17x16x23": lambda: box_system(17, 16, 23, jitter=0.2, sigma_E=1.0, nu_range=(0.25, 0.40), seed=3),
+    "grid8_33x31x33": lambda: box_system(33, 31, 33),
+    "grid4_41x39x40": lambda: box_system(41, 39, 40),
+}
+
+
+@pytest.mark.parametrize("name", list(SYSTEMS))
+@pytest.mark.parametrize("mode", [0, 1])
+def test_one_launch_cg_matches_oracle(name, mode):
+    m = SYSTEMS[name]()
+    m.set_iter(20000)
+    ref = Oracle(m.copy()).solve(coloured=1)
+    m.Iarray[41] = mode
+    with GpuSolver() as s:
+        rec = s.solve(m)
+        info = s.last_solve_info()
+        first = m.X.copy()
+        m.X[:] = 0.0
+        again = s.solve_resident(m.B, m.X, m.Iarray, m.Rarray)
+    assert rec["error"] == ref["error"] == 0
+    assert info["kernels"] <= 4  # the loop is one launch
+    assert abs(rec["iter"] - ref["iter"]) <= 2
+    # both stop with residuals at 1e-8: the parity bound of the solutions
+    assert np.linalg.norm(first - ref["X"]) <= 1e-8 * np.linalg.norm(ref["X"])
+    assert info["true_resid"] < 1e-8
+    assert again["iter"] == rec["iter"] and np.array_equal(first, m.X)
+
+
+def test_recycled_preconditioner_is_not_taken_for_the_matrix():
+    """A recycled SSOR (flag 97 consumed without a rebuild) holds older values than A."""
+    m = box_system(9, 8, 10, jitter=0.2, sigma_E=1.0, nu_range=(0.25, 0.40), seed=11)
+    m.set_iter(20000)
+    with GpuSolver() as s:
+        s.solve(m)
+        for a in (m.D, m.AL, m.AU):
+            a *= 1.7
+        m.X[:] = 0.0
+        m.Iarray[96] = 1  # new values, recycled preconditioner
+        rec = s.solve(m)
+        info = s.last_solve_info()
+    assert info["kernels"] > rec["iter"]  # the colour launches
+    x = m.X.copy()
+    r = m.to_scipy() @ x - m.B
+    assert rec["error"] == 0 and np.linalg.norm(r) <= 1e-8 * np.linalg.norm(m.B)
+
+
+@pytest.mark.parametrize("maxit", [0, 1, 49, 50, 51])
+def test_iteration_limit_and_refresh(maxit):
+    m = box_system(9, 8, 10, jitter=0.2, sigma_E=1.0, nu_range=(0.25, 0.40), seed=11)
+    m.set_iter(maxit)
+    m.set_resid(1e-14)
+    ref = Oracle(m.copy()).solve(coloured=1)
+    with GpuSolver() as s:
+        rec = s.solve(m)
+    assert rec["error"] == ref["error"] and rec["iter"] == ref["iter"]
+    assert np.linalg.norm(m.X - ref["X"]) <= 1e-9 * max(np.linalg.norm(ref["X"]), 1e-300)
