@@ -59,15 +59,27 @@ struct PersistSweep {
   int stride;
 };
 
+// The fused sweeps' vectors in colour-position order.
+struct SsorVecs {
+  const double *alu;  // diagonal LU, entry e of position i at alu[e * n + i]
+  int n;
+  double *r, *g, *p, *q, *h;
+  double2 *zu;        // per position z and v (backward sweep) or u (forward): 3 double2
+};
+
 struct PersistArgs {
   PersistSweep lo, up;
   SellView<double> A;
-  const double *alu;        // diagonal LU, entry e of position i at alu[e * n + i]
+  SsorVecs v;
+  const double *alu;        // block ILU: LU and nodes in the order of the forward levels
   const int *perm, *iperm;  // position -> node and back
+  const double *alu_b;      // and of the backward levels, z in node order, the number of
+  const int *perm_b;        // backward levels
+  double *pz;
+  int nback;
   const double *b;          // node order
   double *x, *r;            // node order: x in and out, r out
-  double *px, *pr, *pg, *pp, *pq, *ph;  // position order
-  double2 *zu;              // per position z and v (backward sweep) or u (forward): 3 double2
+  double *px, *pr, *pp, *pq;  // position order (block ILU: node order)
   CgState *st;
   const CgParams *prm;
   double *parts;            // 3 x gridDim.x partial sums
@@ -169,31 +181,66 @@ __device__ __forceinline__ T ld_row(const T *p) {
   else return *p;
 }
 
+// A warp's slices one after another, as descriptors (first slot, slots, first row,
+// step << 6 | rows) with kPEnd in w after the last: from its list,
+struct ListCursor {
+  const int4 *items;
+  int steps;
+  __device__ __forceinline__ int4 next() {
+    const int4 it = __ldg(items);
+    if (it.w != kPEnd) items++;
+    return it;
+  }
+};
+// or every nw-th slice of the groups [g0, g1) (in reverse), where the team that takes a
+// system is not known beforehand.  desc has the slices' descriptors without their steps.
+struct GroupCursor {
+  const int4 *desc;
+  const int *gs;
+  int g0, steps, back, warp, nw, c, s, end;
+  __device__ __forceinline__ void open() {
+    const int g = back ? g0 + steps - 1 - c : g0 + c;
+    s = __ldg(gs + g) + warp;
+    end = __ldg(gs + g + 1);
+  }
+  __device__ __forceinline__ GroupCursor(const int4 *desc_, const int *gs_, int g0_, int g1_, bool back_, int warp_,
+                                         int nw_)
+      : desc(desc_), gs(gs_), g0(g0_), steps(g1_ - g0_), back(back_), warp(warp_), nw(nw_), c(0), s(0), end(0) {
+    if (steps > 0) open();
+  }
+  __device__ __forceinline__ int4 next() {
+    while (c < steps && s >= end)
+      if (++c < steps) open();
+    if (c >= steps) return make_int4(0, 0, 0, kPEnd);
+    int4 it = __ldg(desc + s);
+    it.w |= c << 6;
+    s += nw;
+    return it;
+  }
+};
+
 // One sweep, MODE 0 backward, 1 forward on the direction, 2 forward from r (start and
 // refresh): the colours in turn, a barrier between them.  K lanes per row; lane c < 3 of
 // a row (MODE 1, K >= 8: of each half of its lanes) carries component c of its vectors.
 // The columns of the slice whose turn is next are loaded before the barrier, so that
 // what follows it is one round of loads: blocks, diagonal LU, own vectors, gathers.
-template <int K, int MODE, bool CLUSTER>
-__device__ __forceinline__ double persist_sweep(const PersistArgs &a, PersistShared &sh, unsigned &target, int w,
-                                                double beta, bool first) {
+template <int K, int MODE, bool CLUSTER, class Cursor, class Barrier>
+__device__ __forceinline__ double ssor_sweep(const SsorVecs &a, const double *val, const int *cols, Cursor cur,
+                                             Barrier barrier, double beta, bool first) {
   constexpr int U = 2;                          // slots taken together (4: more registers, no faster)
   constexpr bool HALVES = MODE == 1 && K >= 8;  // a row's upper lanes end with the sums over z, the lower over u
   const int lane = threadIdx.x & 31;
   const int sub = lane & (K - 1), roff = lane / K;
   const bool up = HALVES && (sub & (K / 2)) != 0;
   const int cc = HALVES ? sub & (K / 2 - 1) : sub, c0 = min(cc, 2);
-  const PersistSweep S = MODE == 0 ? a.up : a.lo;
-  const int4 *items = S.items + size_t(w) * S.stride;
   const size_t n = size_t(a.n);
   double dot = 0.0;
-  int4 it = __ldg(items), nx = __ldg(items + 1);
-  items += 2;
+  int4 it = cur.next(), nx = cur.next();
   int col[U];
 #pragma unroll
-  for (int u = 0; u < U; u++) col[u] = u < it.y ? __ldg(S.col + (it.x + u) * 32 + lane) : 0;
-  for (int c = 0; c < a.ncolor; c++) {
-    if (c) persist_barrier<CLUSTER>(a, sh, target);
+  for (int u = 0; u < U; u++) col[u] = u < it.y ? __ldg(cols + (it.x + u) * 32 + lane) : 0;
+  for (int c = 0; c < cur.steps; c++) {
+    if (c) barrier();
     while ((it.w >> 6) == c) {
       const bool act = roff < (it.w & 63);
       const int row = it.z + (act ? roff : 0), i3 = 3 * row;
@@ -206,25 +253,25 @@ __device__ __forceinline__ double persist_sweep(const PersistArgs &a, PersistSha
       const double *own = reinterpret_cast<const double *>(a.zu + 3 * size_t(row));
       if (MODE == 1) {
         o0 = __ldcg(own + 3), o1 = __ldcg(own + 4), o2 = __ldcg(own + 5);
-        f0 = __ldcg(a.pg + i3 + c0);
+        f0 = __ldcg(a.g + i3 + c0);
         if (HALVES) {
-          if (!first) f1 = __ldcg((up ? a.pq : a.ph) + i3 + c0);
+          if (!first) f1 = __ldcg((up ? a.q : a.h) + i3 + c0);
           if (up) {
             f2 = __ldcg(own + c0);
-            if (!first) f3 = __ldcg(a.pp + i3 + c0);
+            if (!first) f3 = __ldcg(a.p + i3 + c0);
           }
         } else {
           f2 = __ldcg(own + c0);
           if (!first) {
-            f1 = __ldcg(a.ph + i3 + c0);
-            f3 = __ldcg(a.pp + i3 + c0);
-            f4 = __ldcg(a.pq + i3 + c0);
+            f1 = __ldcg(a.h + i3 + c0);
+            f3 = __ldcg(a.p + i3 + c0);
+            f4 = __ldcg(a.q + i3 + c0);
           }
         }
       } else {
-        const double *src = (MODE == 0 ? a.pg : a.pr) + i3;
+        const double *src = (MODE == 0 ? a.g : a.r) + i3;
         o0 = __ldcg(src), o1 = __ldcg(src + 1), o2 = __ldcg(src + 2);
-        if (MODE == 0) f0 = __ldcg(a.pr + i3 + c0);
+        if (MODE == 0) f0 = __ldcg(a.r + i3 + c0);
       }
       double l[3] = {0.0, 0.0, 0.0}, m[3] = {0.0, 0.0, 0.0};  // sums over u (z when MODE 0), and over z
       for (int s = 0; s < it.y; s += U) {
@@ -241,7 +288,7 @@ __device__ __forceinline__ double persist_sweep(const PersistArgs &a, PersistSha
             if (MODE != 2) ga[u] = ld_row<CLUSTER>(g);
             gb[u] = ld_row<CLUSTER>(g + 1);
             if (MODE != 0) gd[u] = ld_row<CLUSTER>(g + 2);
-            const double *b = S.val + size_t(it.x + s + u) * 288 + lane;
+            const double *b = val + size_t(it.x + s + u) * 288 + lane;
 #pragma unroll
             for (int e = 0; e < 9; e++) v[u][e] = __ldcs(b + 32 * e);
           }
@@ -251,7 +298,7 @@ __device__ __forceinline__ double persist_sweep(const PersistArgs &a, PersistSha
         const int slot = more ? it.x + s + U : nx.x, left = more ? nu - U : nx.y;
 #pragma unroll
         for (int u = 0; u < U; u++)
-          if (u < left) col[u] = __ldg(S.col + (slot + u) * 32 + lane);
+          if (u < left) col[u] = __ldg(cols + (slot + u) * 32 + lane);
 #pragma unroll
         for (int u = 0; u < U; u++)
           if (u < nu) {
@@ -267,7 +314,7 @@ __device__ __forceinline__ double persist_sweep(const PersistArgs &a, PersistSha
       if (it.y == 0) {
 #pragma unroll
         for (int u = 0; u < U; u++)
-          if (u < nx.y) col[u] = __ldg(S.col + (nx.x + u) * 32 + lane);
+          if (u < nx.y) col[u] = __ldg(cols + (nx.x + u) * 32 + lane);
       }
       if (HALVES) {
 #pragma unroll
@@ -302,14 +349,14 @@ __device__ __forceinline__ double persist_sweep(const PersistArgs &a, PersistSha
           dot += f0 * xc;
         } else if (MODE == 2) {
           *uo = xc;
-          a.pg[i] = cc == 0 ? e0 : cc == 1 ? e1 : e2;
+          a.g[i] = cc == 0 ? e0 : cc == 1 ? e1 : e2;
         } else if (HALVES) {
           const double t = up ? f0 + lc : f0 - lc;  // g + L z, or g - L u
           const double tn = first ? t : t + beta * f1;
-          (up ? a.pq : a.ph)[i] = tn;
+          (up ? a.q : a.h)[i] = tn;
           if (up) {
             const double pn = first ? f2 : f2 + beta * f3;
-            a.pp[i] = pn;
+            a.p[i] = pn;
             dot += pn * tn;
           } else {
             *uo = xc;
@@ -323,21 +370,37 @@ __device__ __forceinline__ double persist_sweep(const PersistArgs &a, PersistSha
             hn = hn + beta * f1;
           }
           *uo = xc;
-          a.pp[i] = pn;
-          a.pq[i] = qn;
-          a.ph[i] = hn;
+          a.p[i] = pn;
+          a.q[i] = qn;
+          a.h[i] = hn;
           dot += pn * qn;
         }
       }
       it = nx;
-      nx = __ldg(items);
-      if (nx.w != kPEnd) items++;
+      nx = cur.next();
     }
   }
   return dot;
 }
 
-// r = b - A x from x in node order, r in position order; |r|^2 or (BB) |b|^2.
+template <int K, int MODE, bool CLUSTER>
+__device__ __forceinline__ double persist_sweep(const PersistArgs &a, PersistShared &sh, unsigned &target, int w,
+                                                double beta, bool first) {
+  const PersistSweep S = MODE == 0 ? a.up : a.lo;
+  return ssor_sweep<K, MODE, CLUSTER>(a.v, S.val, S.col, ListCursor{S.items + size_t(w) * S.stride, a.ncolor},
+                                      [&] { persist_barrier<CLUSTER>(a, sh, target); }, beta, first);
+}
+
+// Descriptors of a layout's slices for GroupCursor.
+static __global__ void slice_desc_kernel(const int *__restrict__ slot0, const int *__restrict__ len,
+                                         const int *__restrict__ row0, const int *__restrict__ nrows, int n,
+                                         int4 *__restrict__ desc) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    desc[i] = make_int4(slot0[i], len[i], row0[i], nrows[i]);
+}
+
+// r = b - A x from x in node order, r in position order (node order without iperm);
+// |r|^2 or (BB) |b|^2.
 template <bool BB>
 __device__ __forceinline__ double persist_resid(const PersistArgs &a) {
   const int lane = threadIdx.x & 31;
@@ -354,24 +417,19 @@ __device__ __forceinline__ double persist_resid(const PersistArgs &a) {
       y0 = b0 - y0;
       y1 = b1 - y1;
       y2 = b2 - y2;
-      const int i3 = 3 * a.iperm[row];
-      a.pr[i3] = y0;
-      a.pr[i3 + 1] = y1;
-      a.pr[i3 + 2] = y2;
+      double *r = a.pr + 3 * (a.iperm ? a.iperm[row] : row);
+      r[0] = y0;
+      r[1] = y1;
+      r[2] = y2;
       acc += BB ? b0 * b0 + b1 * b1 + b2 * b2 : y0 * y0 + y1 * y1 + y2 * y2;
     }
   }
   return acc;
 }
 
-template <int K, bool CLUSTER>
-__global__ void __launch_bounds__(32 * persist_warps<K>(), 1) cg_ssor_persist_kernel(const PersistArgs a) {
-  __shared__ PersistShared sh;
-  const int tid = threadIdx.x, warp = tid >> 5;
-  const int w = warp * gridDim.x + blockIdx.x;  // this warp's list: neighbouring slices on different SMs
-  const int gt = blockIdx.x * blockDim.x + tid, nt = gridDim.x * blockDim.x;
-  unsigned target = 0;
-  if (tid == 0) {
+// The CG's scalars at the start of a solve, one replica per CTA.
+__device__ __forceinline__ void persist_begin(const PersistArgs &a, PersistShared &sh) {
+  if (threadIdx.x == 0) {
     CgState &st = sh.st;
     st.rho = st.rho1 = st.alpha = st.beta = st.pq = st.rr = 0.0;
     st.bnrm2 = st.resid = st.rr_true = 0.0;
@@ -398,28 +456,75 @@ __global__ void __launch_bounds__(32 * persist_warps<K>(), 1) cg_ssor_persist_ke
     sh.dead = 0;
   }
   __syncthreads();
+}
+
+// ||b||^2, and whether the loop runs at all.
+__device__ __forceinline__ void persist_bnrm(PersistShared &sh, double bb) {
+  if (threadIdx.x == 0) {
+    CgState &st = sh.st;
+    st.bnrm2 = bb;
+    if (bb == 0.0) {
+      st.zero_rhs = 1;
+      st.done = 1;
+    }
+    if (st.maxit <= 0) st.done = 1;
+  }
+  __syncthreads();
+}
+
+// The residual recomputed from b - A x (every 50th iteration, or below the tolerance).
+__device__ __forceinline__ void persist_true_resid(PersistShared &sh, double rr, bool refresh) {
+  if (threadIdx.x == 0) {
+    CgState &st = sh.st;
+    st.rr = rr;
+    st.resid = sqrt(rr / st.bnrm2);
+    if (refresh) record_resid(&st);
+    if (st.resid <= st.tol) {
+      st.done = 1;
+      st.converged = 1;
+    }
+  }
+}
+
+// The end of an iteration.
+__device__ __forceinline__ void persist_ctl(PersistShared &sh) {
+  if (threadIdx.x == 0) {
+    loop_ctl(&sh.st, 0, 0);
+    if (sh.dead) sh.st.done = 1;
+  }
+  __syncthreads();
+}
+
+// The state out, after the last use of the vectors.
+__device__ __forceinline__ void persist_end(const PersistArgs &a, PersistShared &sh) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (sh.dead) {
+      sh.st.error = HECMW33_ERR_TIMEOUT;
+      sh.st.done = 1;
+    }
+    *a.st = sh.st;
+  }
+}
+
+template <int K, bool CLUSTER>
+__global__ void __launch_bounds__(32 * persist_warps<K>(), 1) cg_ssor_persist_kernel(const PersistArgs a) {
+  __shared__ PersistShared sh;
+  const int tid = threadIdx.x, warp = tid >> 5;
+  const int w = warp * gridDim.x + blockIdx.x;  // this warp's list: neighbouring slices on different SMs
+  const int gt = blockIdx.x * blockDim.x + tid, nt = gridDim.x * blockDim.x;
+  unsigned target = 0;
+  persist_begin(a, sh);
   // x in position order; z and u start at zero (padding blocks gather position 0)
   for (int i = gt; i < a.n; i += nt) {
     const int node = a.perm[i];
 #pragma unroll
     for (int c = 0; c < 3; c++) {
       a.px[3 * i + c] = a.x[3 * node + c];
-      a.zu[3 * size_t(i) + c] = make_double2(0.0, 0.0);
+      a.v.zu[3 * size_t(i) + c] = make_double2(0.0, 0.0);
     }
   }
   CgState &st = sh.st;
-  {
-    const double bb = persist_sum<CLUSTER>(a, sh, target, persist_resid<true>(a), 0);
-    if (tid == 0) {
-      st.bnrm2 = bb;
-      if (bb == 0.0) {
-        st.zero_rhs = 1;
-        st.done = 1;
-      }
-      if (st.maxit <= 0) st.done = 1;
-    }
-    __syncthreads();
-  }
+  persist_bnrm(sh, persist_sum<CLUSTER>(a, sh, target, persist_resid<true>(a), 0));
   const int n3 = 3 * a.n, n2 = n3 / 2;
   bool restart = true;  // g from r
   while (!st.done) {
@@ -444,9 +549,9 @@ __global__ void __launch_bounds__(32 * persist_warps<K>(), 1) cg_ssor_persist_ke
       const double alpha = st.alpha;
       double rr = 0.0;
       double2 *x2 = reinterpret_cast<double2 *>(a.px), *r2 = reinterpret_cast<double2 *>(a.pr),
-              *g2 = reinterpret_cast<double2 *>(a.pg);
+              *g2 = reinterpret_cast<double2 *>(a.v.g);
       const double2 *p2 = reinterpret_cast<const double2 *>(a.pp), *q2 = reinterpret_cast<const double2 *>(a.pq),
-                    *h2 = reinterpret_cast<const double2 *>(a.ph);
+                    *h2 = reinterpret_cast<const double2 *>(a.v.h);
       for (int i = gt; i < n2; i += nt) {
         double2 x = __ldcg(x2 + i);
         const double2 p = __ldcg(p2 + i);
@@ -471,7 +576,7 @@ __global__ void __launch_bounds__(32 * persist_warps<K>(), 1) cg_ssor_persist_ke
         if (!refresh) {
           const double r = -alpha * __ldcg(a.pq + i) + __ldcg(a.pr + i);
           a.pr[i] = r;
-          a.pg[i] = -alpha * __ldcg(a.ph + i) + __ldcg(a.pg + i);
+          a.v.g[i] = -alpha * __ldcg(a.v.h + i) + __ldcg(a.v.g + i);
           rr += r * r;
         }
       }
@@ -489,23 +594,10 @@ __global__ void __launch_bounds__(32 * persist_warps<K>(), 1) cg_ssor_persist_ke
         for (int c = 0; c < 3; c++) a.x[3 * node + c] = __ldcg(a.px + 3 * i + c);
       }
       persist_barrier<CLUSTER>(a, sh, target);
-      const double rr = persist_sum<CLUSTER>(a, sh, target, persist_resid<false>(a), 2);
-      if (tid == 0) {
-        st.rr = rr;
-        st.resid = sqrt(rr / st.bnrm2);
-        if (refresh) record_resid(&st);
-        if (st.resid <= st.tol) {
-          st.done = 1;
-          st.converged = 1;
-        }
-      }
+      persist_true_resid(sh, persist_sum<CLUSTER>(a, sh, target, persist_resid<false>(a), 2), refresh);
       restart = true;
     }
-    if (tid == 0) {
-      loop_ctl(&st, 0, 0);
-      if (sh.dead) st.done = 1;
-    }
-    __syncthreads();
+    persist_ctl(sh);
   }
   if (!sh.dead && !st.zero_rhs) {
     for (int i = gt; i < a.n; i += nt) {
@@ -517,13 +609,189 @@ __global__ void __launch_bounds__(32 * persist_warps<K>(), 1) cg_ssor_persist_ke
       }
     }
   }
-  if (blockIdx.x == 0 && tid == 0) {
-    if (sh.dead) {
-      st.error = HECMW33_ERR_TIMEOUT;
-      st.done = 1;
+  persist_end(a, sh);
+  if constexpr (CLUSTER) persist_barrier<true>(a, sh, target);
+}
+
+// ---- block ILU ----------------------------------------------------------------------
+// The CG with a block ILU(p) preconditioner, whose levels take the place of the colours:
+// its triangles are not A's, so q = A p is a pass of its own, and the vectors stay in
+// node order.  A level of a lexicographically numbered box has a few hundred rows, so the
+// solve is the latency of its two chains of levels: at 40^3 elements (281 + 281) an
+// iteration took 4.5 ms as one launch per level and takes 1.68 ms here, 3 us a level of
+// which the barrier with the stores before it and the first load after it are 1.65.
+//
+// One direction: forward z = LU^-1 (r - L z), backward z -= LU^-1 (U z) with RHO = r.z.
+template <int K, bool BACK, bool CLUSTER>
+__device__ __forceinline__ double persist_levels(const PersistArgs &a, PersistShared &sh, unsigned &target, int w) {
+  constexpr int U = 2;
+  const int lane = threadIdx.x & 31;
+  const int sub = lane & (K - 1), roff = lane / K;
+  const PersistSweep S = BACK ? a.up : a.lo;
+  const double *alu = BACK ? a.alu_b : a.alu;
+  const int *perm = BACK ? a.perm_b : a.perm;
+  const int nstep = BACK ? a.nback : a.ncolor;
+  const int4 *items = S.items + size_t(w) * S.stride;
+  const size_t n = size_t(a.n);
+  double dot = 0.0;
+  int4 it = __ldg(items), nx = __ldg(items + 1);
+  items += 2;
+  int col[U];
+#pragma unroll
+  for (int u = 0; u < U; u++) col[u] = u < it.y ? __ldg(S.col + (it.x + u) * 32 + lane) : 0;
+  int node = it.w == kPEnd ? 0 : __ldg(perm + it.z + (roff < (it.w & 63) ? roff : 0));
+  for (int c = 0; c < nstep; c++) {
+    if (c) persist_barrier<CLUSTER>(a, sh, target);
+    while ((it.w >> 6) == c) {
+      const bool act = roff < (it.w & 63);
+      const int row = it.z + (act ? roff : 0), i3 = 3 * node;
+      const double *lu = alu + row;
+      const double a0 = __ldcs(lu), a1 = __ldcs(lu + n), a2 = __ldcs(lu + 2 * n);
+      const double a3 = __ldcs(lu + 3 * n), a4 = __ldcs(lu + 4 * n), a5 = __ldcs(lu + 5 * n);
+      const double a6 = __ldcs(lu + 6 * n), a7 = __ldcs(lu + 7 * n), a8 = __ldcs(lu + 8 * n);
+      const double *own = (BACK ? a.pz : a.r) + i3;
+      const double o0 = __ldcg(own), o1 = __ldcg(own + 1), o2 = __ldcg(own + 2);
+      const double rc = BACK ? __ldcg(a.r + i3 + min(sub, 2)) : 0.0;
+      double l[3] = {0.0, 0.0, 0.0};
+      const int next = nx.w == kPEnd ? 0 : __ldg(perm + nx.z + (roff < (nx.w & 63) ? roff : 0));
+      for (int s = 0; s < it.y; s += U) {
+        const int nu = it.y - s;
+        double x[U][3], v[U][9];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+#pragma unroll
+          for (int j = 0; j < 3; j++) x[u][j] = 0.0;
+#pragma unroll
+          for (int e = 0; e < 9; e++) v[u][e] = 0.0;
+          if (u < nu) {
+            const double *g = a.pz + 3 * size_t(col[u]);
+#pragma unroll
+            for (int j = 0; j < 3; j++) x[u][j] = ld_row<CLUSTER>(g + j);
+            const double *b = S.val + size_t(it.x + s + u) * 288 + lane;
+#pragma unroll
+            for (int e = 0; e < 9; e++) v[u][e] = __ldcs(b + 32 * e);
+          }
+        }
+        const bool more = nu > U;
+        const int slot = more ? it.x + s + U : nx.x, left = more ? nu - U : nx.y;
+#pragma unroll
+        for (int u = 0; u < U; u++)
+          if (u < left) col[u] = __ldg(S.col + (slot + u) * 32 + lane);
+#pragma unroll
+        for (int u = 0; u < U; u++)
+          if (u < nu) {
+#pragma unroll
+            for (int i = 0; i < 3; i++)
+              l[i] = fma(v[u][3 * i + 2], x[u][2], fma(v[u][3 * i + 1], x[u][1], fma(v[u][3 * i], x[u][0], l[i])));
+          }
+      }
+      if (it.y == 0) {
+#pragma unroll
+        for (int u = 0; u < U; u++)
+          if (u < nx.y) col[u] = __ldg(S.col + (nx.x + u) * 32 + lane);
+      }
+#pragma unroll
+      for (int o = K / 2; o > 0; o >>= 1) {
+#pragma unroll
+        for (int j = 0; j < 3; j++) l[j] += __shfl_xor_sync(0xffffffffu, l[j], o);
+      }
+      double x1 = BACK ? l[0] : o0 - l[0], x2 = BACK ? l[1] : o1 - l[1], x3 = BACK ? l[2] : o2 - l[2];
+      x2 = x2 - a3 * x1;
+      x3 = x3 - a6 * x1 - a7 * x2;
+      x3 = a8 * x3;
+      x2 = a4 * (x2 - a5 * x3);
+      x1 = a0 * (x1 - a2 * x3 - a1 * x2);
+      if (act && sub < 3) {
+        double zc = sub == 0 ? x1 : sub == 1 ? x2 : x3;
+        if (BACK) {
+          zc = (sub == 0 ? o0 : sub == 1 ? o1 : o2) - zc;
+          dot += rc * zc;
+        }
+        a.pz[i3 + sub] = zc;
+      }
+      it = nx;
+      node = next;
+      nx = __ldg(items);
+      if (nx.w != kPEnd) items++;
     }
-    *a.st = st;
   }
+  return dot;
+}
+
+// q = A p over the grid with the partial of p.q.
+__device__ __forceinline__ double persist_product(const PersistArgs &a) {
+  const int lane = threadIdx.x & 31;
+  const int nw = (gridDim.x * blockDim.x) >> 5;
+  double acc = 0.0;
+  for (int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; s < a.A.nslices; s += nw) {
+    const bool active = lane < a.A.nrows[s];
+    const int row = a.A.row0[s] + lane;
+    const int len = active ? a.A.rowlen[s * 32 + lane] : 0;
+    double y0 = 0.0, y1 = 0.0, y2 = 0.0;
+    row_gemv<double, double, 1, false, true>(a.A, s, lane, len, a.pp, y0, y1, y2);
+    if (active) {
+      a.pq[3 * row] = y0;
+      a.pq[3 * row + 1] = y1;
+      a.pq[3 * row + 2] = y2;
+      acc += __ldcg(a.pp + 3 * row) * y0 + __ldcg(a.pp + 3 * row + 1) * y1 + __ldcg(a.pp + 3 * row + 2) * y2;
+    }
+  }
+  return acc;
+}
+
+template <int K, bool CLUSTER>
+__global__ void __launch_bounds__(32 * persist_warps<K>(), 1) cg_ilu_persist_kernel(const PersistArgs a) {
+  __shared__ PersistShared sh;
+  const int tid = threadIdx.x;
+  const int w = (tid >> 5) * gridDim.x + blockIdx.x;
+  const int gt = blockIdx.x * blockDim.x + tid, nt = gridDim.x * blockDim.x;
+  unsigned target = 0;
+  persist_begin(a, sh);
+  const int n3 = 3 * a.n;
+  for (int i = gt; i < n3; i += nt) a.pz[i] = 0.0;  // padding blocks gather node 0
+  persist_bnrm(sh, persist_sum<CLUSTER>(a, sh, target, persist_resid<true>(a), 0));
+  CgState &st = sh.st;
+  while (!st.done) {
+    if (tid == 0) st.guard++;
+    persist_levels<K, false, CLUSTER>(a, sh, target, w);
+    persist_barrier<CLUSTER>(a, sh, target);
+    const double rho = persist_sum<CLUSTER>(a, sh, target, persist_levels<K, true, CLUSTER>(a, sh, target, w), 0);
+    if (tid == 0) fin_rho(&st, rho);
+    __syncthreads();
+    if (st.done) break;
+    const bool first = st.iter == 1;
+    const double beta = st.beta;
+    for (int i = gt; i < n3; i += nt) {
+      const double z = __ldcg(a.pz + i);
+      a.pp[i] = first ? z : z + beta * __ldcg(a.pp + i);
+    }
+    persist_barrier<CLUSTER>(a, sh, target);
+    const double pq = persist_sum<CLUSTER>(a, sh, target, persist_product(a), 1);
+    if (tid == 0) fin_pq(&st, pq);
+    __syncthreads();
+    if (st.done) break;
+    const bool refresh = (st.iter % st.nrecompute) == 0;
+    const double alpha = st.alpha;
+    double rr = 0.0;
+    for (int i = gt; i < n3; i += nt) {
+      a.x[i] = alpha * __ldcg(a.pp + i) + __ldcg(a.x + i);
+      if (!refresh) {
+        const double r = -alpha * __ldcg(a.pq + i) + __ldcg(a.r + i);
+        a.r[i] = r;
+        rr += r * r;
+      }
+    }
+    rr = persist_sum<CLUSTER>(a, sh, target, rr, 2);
+    if (!refresh) {
+      if (tid == 0) fin_rr(&st, rr);
+      __syncthreads();
+    }
+    if (refresh || st.recompute)
+      persist_true_resid(sh, persist_sum<CLUSTER>(a, sh, target, persist_resid<false>(a), 1), refresh);
+    // r (and x) are complete at a barrier before the next sweep gathers or overwrites
+    persist_ctl(sh);
+  }
+  persist_end(a, sh);
   if constexpr (CLUSTER) persist_barrier<true>(a, sh, target);
 }
 

@@ -1040,7 +1040,7 @@ void setup_ssor(Solver &S, Precond &P, int ncolor_in, double sigma, bool symboli
 // (FORM_ILU0_33), p = 1, 2 on the fill pattern of FORM_ILU1_33 / FORM_ILU2_33.  The
 // factorisation runs on the host from the resident values; the forward and backward
 // solves run on the device in level schedules of the factor pattern.
-void setup_bilu(Solver &S, int level, double sigma, bool symbolic) {
+void setup_bilu(Solver &S, int level, double sigma, bool symbolic, bool cg) {
   Precond &P = S.pc;
   const Profile prof0{S.N, S.indexL.data(), S.itemL.data(), S.indexU.data(), S.itemU.data()};
   if (symbolic) {
@@ -1049,10 +1049,11 @@ void setup_bilu(Solver &S, int level, double sigma, bool symbolic) {
     std::vector<int> ord_f, lev_f, ord_b, lev_b;
     level_schedule(prof, true, ord_f, lev_f);
     level_schedule(prof, false, ord_b, lev_b);
+    const int lanes = cg ? ssor_lanes(S.N, int(lev_f.size()) - 1, S.nsm) : sweep_lanes();
     if (level == 0 && !host_layouts()) {
       // the matrix's own pattern: the shapes from the rows' counts, the blocks placed
       // on the device from the resident profile (fill_ordered_kernel)
-      const int N = S.N, lanes = sweep_lanes();
+      const int N = S.N;
       const size_t nn = static_cast<size_t>(N);
       std::vector<int> cl(nn), cu(nn);
       for (int q = 0; q < N; q++) {
@@ -1114,8 +1115,8 @@ void setup_bilu(Solver &S, int level, double sigma, bool symbolic) {
         }
       }
       SellLayout lo, up;
-      build_sell(lower, lev_f, lo, sweep_lanes());
-      build_sell(upper, lev_b, up, sweep_lanes());
+      build_sell(lower, lev_f, lo, lanes);
+      build_sell(upper, lev_b, up, lanes);
       P.lo.upload(lo, S.stream);
       P.up.upload(up, S.stream);
       P.perm_fwd.upload(ord_f, S.stream);
@@ -1194,7 +1195,7 @@ void precond_setup(Solver &S, int precond, int ncolor_in, double sigma, int *Iar
   P.ncolor_in = ncolor_in;
   if (kind == 1) setup_ssor(S, P, ncolor_in, sigma, symbolic, false, Iarray[1] == 1);
   else if (kind == 3) diag_alu(S, P.alu_fwd, S.raw.p, nullptr, sigma, 0);
-  else setup_bilu(S, level, sigma, symbolic);
+  else setup_bilu(S, level, sigma, symbolic, Iarray[1] == 1);
   int err = 0;
   H33_CUDA(cudaMemcpyAsync(&err, S.d_err.p, sizeof(int), cudaMemcpyDeviceToHost, S.stream));
   S.sync();
@@ -1804,13 +1805,15 @@ float run_cg(Solver &S, int iterpremax, double tol, int maxit, int *kernels, int
   return ms;
 }
 
-// Whether the plain FP64 CG of this solve can run as cg_ssor_persist_kernel: SSOR in the
-// colour layout with SIGMA_DIAG = 1, built from the very values of the resident matrix
-// (a recycled preconditioner is not A's own triangles any more).
+// Whether the plain FP64 CG of this solve can run in one launch: any block ILU
+// (cg_ilu_persist_kernel), or SSOR in the colour layout with SIGMA_DIAG = 1 built from the
+// very values of the resident matrix (cg_ssor_persist_kernel; a recycled preconditioner
+// is not A's own triangles any more).
 bool persist_ok(const Solver &S, int iterpremax) {
   const Precond &P = S.pc;
-  return P.valid && P.kind == 1 && P.pos_cols && iterpremax == 1 && P.sigma == 1.0 &&
-         P.values_version == S.values_version;
+  if (!P.valid || iterpremax != 1) return false;
+  if (P.kind == 10) return true;
+  return P.kind == 1 && P.pos_cols && P.sigma == 1.0 && P.values_version == S.values_version;
 }
 
 template <int K, bool CLUSTER>
@@ -1832,17 +1835,18 @@ void persist_config(Solver &S, int grid, cudaLaunchConfig_t &cfg, cudaLaunchAttr
 }
 
 // CTAs of the launch, negative for one cluster of that many: a cluster of 16 (of 8 where
-// the device cannot place 16) while a colour's rows fit its warps at 16 lanes a row once
-// (384 rows; 69 us an iteration against 89 us on the whole grid at 143 rows a colour),
-// else a CTA per SM.
+// the device cannot place 16) while the rows of a colour or level are no more than its
+// warps, else a CTA per SM.  Measured on the cluster / the grid (us an iteration): SSOR
+// 22 rows a colour 60 / 86, 143 rows 69 / 89; ILU(0) 15 rows a level 313 / 417, 61 rows
+// 1291 / 1601, 160 rows 1137 / 1281, 245 rows 1805 / 1680.
 template <int K>
-int persist_grid(Solver &S, int rows) {
+int persist_grid(Solver &S, bool ilu, int rows) {
   constexpr int W = persist_warps<K>();
   if constexpr (K == 16) {
-    auto kern = cg_ssor_persist_kernel<K, true>;
+    auto kern = ilu ? cg_ilu_persist_kernel<K, true> : cg_ssor_persist_kernel<K, true>;
     H33_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     for (int c : {16, 8}) {
-      if (rows > 2 * c * W) break;
+      if (rows > c * W) break;
       cudaLaunchConfig_t cfg;
       cudaLaunchAttribute attr[1];
       persist_config<K, true>(S, c, cfg, attr);
@@ -1852,7 +1856,8 @@ int persist_grid(Solver &S, int rows) {
     }
   }
   int per_sm = 0;
-  H33_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cg_ssor_persist_kernel<K, false>, 32 * W, 0));
+  H33_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+      &per_sm, ilu ? cg_ilu_persist_kernel<K, false> : cg_ssor_persist_kernel<K, false>, 32 * W, 0));
   if (per_sm < 1) throw Failure(HECMW33_ERR_CUDA, "the persistent CG does not fit an SM");
   return S.nsm;
 }
@@ -1862,12 +1867,12 @@ void persist_plan(Solver &S) {
   PersistPlan &L = S.pp;
   const Precond &P = S.pc;
   if (L.generation == P.generation) return;
-  const int ng = int(P.lo.group_slice.size()) - 1;
-  const int grid = persist_grid<K>(S, S.N / std::max(ng, 1));
+  const int grid = persist_grid<K>(S, P.kind == 10, S.N / std::max(int(P.lo.group_slice.size()) - 1, 1));
   L.cluster = grid < 0;
   L.grid = std::abs(grid);
   const int nw = L.grid * persist_warps<K>();
   auto lists = [&](const DevSell<double> &D, bool reverse, DevArray<int4> &items, int &stride) {
+    const int ng = int(D.group_slice.size()) - 1;
     stride = 2;
     for (int g = 0; g < ng; g++) stride += (D.group_slice[size_t(g) + 1] - D.group_slice[size_t(g)] + nw - 1) / nw;
     DevArray<int> gs;
@@ -1881,10 +1886,13 @@ void persist_plan(Solver &S) {
   };
   lists(P.lo, false, L.lo_items, L.lo_stride);
   lists(P.up, true, L.up_items, L.up_stride);
-  L.iperm.alloc(size_t(S.N));
-  launch_k(S.stream, invert_perm_kernel, S.grid_vec(), kThreads, static_cast<const int *>(P.perm_fwd.p), S.N, L.iperm.p);
-  H33_CUDA(cudaGetLastError());
-  L.zu.alloc(6 * size_t(S.N));
+  if (P.kind == 1) {
+    L.iperm.alloc(size_t(S.N));
+    launch_k(S.stream, invert_perm_kernel, S.grid_vec(), kThreads, static_cast<const int *>(P.perm_fwd.p), S.N,
+             L.iperm.p);
+    H33_CUDA(cudaGetLastError());
+    L.zu.alloc(6 * size_t(S.N));
+  }
   L.parts.alloc(3 * size_t(L.grid));
   L.bar.alloc(2);
   L.generation = P.generation;
@@ -1892,20 +1900,21 @@ void persist_plan(Solver &S) {
 
 template <int K>
 void launch_persist(Solver &S, const PersistArgs &a) {
+  const bool ilu = S.pc.kind == 10;
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute attr[1];
   if constexpr (K == 16) {
     if (S.pp.cluster) {
       persist_config<K, true>(S, S.pp.grid, cfg, attr);
-      H33_CUDA(cudaLaunchKernelEx(&cfg, cg_ssor_persist_kernel<K, true>, a));
+      H33_CUDA(cudaLaunchKernelEx(&cfg, ilu ? cg_ilu_persist_kernel<K, true> : cg_ssor_persist_kernel<K, true>, a));
       return;
     }
   }
   persist_config<K, false>(S, S.pp.grid, cfg, attr);
-  H33_CUDA(cudaLaunchKernelEx(&cfg, cg_ssor_persist_kernel<K, false>, a));
+  H33_CUDA(cudaLaunchKernelEx(&cfg, ilu ? cg_ilu_persist_kernel<K, false> : cg_ssor_persist_kernel<K, false>, a));
 }
 
-// As run_cg for the plain FP64 CG, the whole solve in one cg_ssor_persist_kernel.
+// As run_cg for the plain FP64 CG, the whole solve in one launch.
 float run_cg_persist(Solver &S, double tol, int maxit, int *kernels) {
   const Precond &P = S.pc;
   switch (P.lo.lanes) {
@@ -1925,7 +1934,7 @@ float run_cg_persist(Solver &S, double tol, int maxit, int *kernels) {
   h.lanczos_cap = S.lanczos_on ? int(S.lanczos_buf.n / 2) : 0;
   h.rhist = S.rhist_on ? S.rhist_buf.p : nullptr;
   h.rhist_cap = S.rhist_on ? int(S.rhist_buf.n) : 0;
-  PersistArgs a;
+  PersistArgs a = {};
   a.lo = PersistSweep{P.lo.val.p, P.lo.col.p, L.lo_items.p, L.lo_stride};
   a.up = PersistSweep{P.up.val.p, P.up.col.p, L.up_items.p, L.up_stride};
   a.A = S.A.view();
@@ -1935,14 +1944,20 @@ float run_cg_persist(Solver &S, double tol, int maxit, int *kernels) {
   a.b = S.b.p;
   a.x = S.x.p;
   a.r = S.r.p;
-  // the solve's work vectors, here in position order
-  a.px = S.w.p;
-  a.pr = S.zp.p;
-  a.pg = S.z.p;
   a.pp = S.p.p;
   a.pq = S.q.p;
-  a.ph = S.zpos.p;
-  a.zu = reinterpret_cast<double2 *>(L.zu.p);
+  if (P.kind == 10) {
+    a.iperm = nullptr;
+    a.pr = S.r.p;
+    a.pz = S.z.p;
+    a.alu_b = P.alu_bwd.p;
+    a.perm_b = P.perm_bwd.p;
+    a.nback = int(P.up.group_slice.size()) - 1;
+  } else {  // the solve's work vectors, here in position order
+    a.px = S.w.p;
+    a.pr = S.zp.p;
+    a.v = SsorVecs{P.alu_fwd.p, S.N, a.pr, S.z.p, a.pp, a.pq, S.zpos.p, reinterpret_cast<double2 *>(L.zu.p)};
+  }
   a.st = S.state.p;
   a.prm = S.params.p;
   a.parts = L.parts.p;

@@ -40,8 +40,8 @@ SYSTEMS = {
     "box_1x1x1": lambda: box_system(1, 1, 1),
     "box_2x1x3": lambda: box_system(2, 1, 3),
     "hubs": hub_system,
-    "cluster_14x14x20": lambda: box_system(14, 14, 20, jitter=0.2, sigma_E=1.0, nu_range=(0.25, 0.40), seed=3),
-    "grid16_17x16x23": lambda: box_system(17, 16, 23, jitter=0.2, sigma_E=1.0, nu_range=(0.25, 0.40), seed=3),
+    "cluster_12x12x17": lambda: box_system(12, 12, 17, jitter=0.2, sigma_E=1.0, nu_range=(0.25, 0.40), seed=3),
+    "grid16_14x14x20": lambda: box_system(14, 14, 20, jitter=0.2, sigma_E=1.0, nu_range=(0.25, 0.40), seed=3),
     "grid8_33x31x33": lambda: box_system(33, 31, 33),
     "grid4_41x39x40": lambda: box_system(41, 39, 40),
 }
@@ -67,6 +67,41 @@ def test_one_launch_cg_matches_oracle(name, mode):
     assert np.linalg.norm(first - ref["X"]) <= 1e-8 * np.linalg.norm(ref["X"])
     assert info["true_resid"] < 1e-8
     assert again["iter"] == rec["iter"] and np.array_equal(first, m.X)
+
+
+@pytest.mark.parametrize("precond", [10, 11])
+@pytest.mark.parametrize("name", ["box_1x1x1", "hubs", "cluster_12x12x17", "grid_43x40x36"])
+def test_one_launch_ilu_cg_matches_oracle(name, precond):
+    if name == "grid_43x40x36":
+        if precond == 11:
+            pytest.skip("the oracle's fill takes minutes")
+        m = box_system(43, 40, 36)
+    else:
+        m = SYSTEMS[name]()
+    m.set_iter(20000)
+    m.set_precond(precond)
+    ref = Oracle(m.copy()).solve(coloured=1)
+    with GpuSolver() as s:
+        rec = s.solve(m)
+        info = s.last_solve_info()
+    assert rec["error"] == ref["error"] == 0 and info["kernels"] <= 4
+    assert abs(rec["iter"] - ref["iter"]) <= 2
+    assert np.linalg.norm(m.X - ref["X"]) <= 1e-8 * np.linalg.norm(ref["X"])
+
+
+def test_handle_that_changes_its_preconditioner():
+    """SSOR, block ILU and SSOR again on one handle: nothing of one plan is left to the next."""
+    m = box_system(9, 8, 10, jitter=0.2, sigma_E=1.0, nu_range=(0.25, 0.40), seed=11)
+    m.set_iter(20000)
+    out = []
+    with GpuSolver() as s:
+        for precond in (1, 10, 1):
+            g = m.copy()
+            g.set_precond(precond)
+            assert s.solve(g)["error"] == 0
+            out.append(g.X)
+    assert np.array_equal(out[0], out[2])
+    assert np.linalg.norm(out[1] - out[0]) <= 1e-7 * np.linalg.norm(out[0])
 
 
 def test_recycled_preconditioner_is_not_taken_for_the_matrix():
