@@ -15,6 +15,8 @@
 //    sums in the same order, so no scalar round-trips through global memory and all
 //    CTAs of a team take the same branches);
 //  * small systems (second queue): each CTA solves one system alone (CTA barriers).
+// With SSOR, one pass and SIGMA_DIAG = 1 a system runs the fused iteration of
+// cg_ssor_persist_kernel (team_solve_fused: no product, its blocks read once).
 // Queues are ordered by decreasing estimated work (longest-first scheduling), so
 // the big systems start first and the small ones fill the gaps.  All vector reads
 // of data written during the launch go through L2 (__ldcg), never the read-only path.
@@ -24,7 +26,7 @@
 
 #include <cooperative_groups.h>
 
-#include "h33_kernels.cuh"
+#include "h33_persist.cuh"
 
 namespace h33 {
 
@@ -49,7 +51,8 @@ struct BatchOut {
 struct BatchArgs {
   SellView<double> A, lo, up;
   const int *lo_gs, *up_gs;  // group g -> slices [gs[g], gs[g+1])
-  const int *perm;           // position -> node (global)
+  const int4 *lo_desc, *up_desc;  // the slices' descriptors (GroupCursor)
+  const int *perm, *iperm;   // position -> node (global) and back
   const double *alu;         // SoA, stride npos
   int npos;
   int kind;                  // 1 SSOR, 3 DIAG
@@ -60,6 +63,9 @@ struct BatchArgs {
   int *queue;                // [0] big, [1] small
   const double *b;
   double *x, *r, *z, *p, *q;
+  double *zpos;              // the sweeps' intermediate in position order (unfused)
+  double *px;                // position order: x, and the fused sweeps' vectors
+  SsorVecs v;
   BatchOut *out;
   double tol;
   int maxit;
@@ -113,7 +119,8 @@ __device__ __forceinline__ double team_sum(Team &t, double v, double *s_warp, do
 
 // r = b - A x over the system's slices (one lane per row); returns this thread's
 // partial of |r|^2 (WITH_RR) or of |b|^2 (WITH_BB).
-template <bool WITH_RR, bool WITH_BB>
+// POS: r in position order.
+template <bool WITH_RR, bool WITH_BB, bool POS = false>
 __device__ __forceinline__ double team_resid(const BatchArgs &a, const BatchSys &sy, const Team &t, const double *x,
                                              double *r) {
   const int lane = threadIdx.x & 31;
@@ -129,9 +136,10 @@ __device__ __forceinline__ double team_resid(const BatchArgs &a, const BatchSys 
       y0 = b0 - y0;
       y1 = b1 - y1;
       y2 = b2 - y2;
-      r[3 * row] = y0;
-      r[3 * row + 1] = y1;
-      r[3 * row + 2] = y2;
+      double *ro = r + 3 * (POS ? a.iperm[row] : row);
+      ro[0] = y0;
+      ro[1] = y1;
+      ro[2] = y2;
       if (WITH_RR) acc += y0 * y0 + y1 * y1 + y2 * y2;
       if (WITH_BB) acc += b0 * b0 + b1 * b1 + b2 * b2;
     }
@@ -170,15 +178,16 @@ __device__ __forceinline__ double team_fwd(const BatchArgs &a, const Team &t, in
     const int row = a.lo.row0[s] + roff;
     const int len = active ? a.lo.rowlen[s * 32 + roff] : 0;
     double a0 = 0.0, a1 = 0.0, a2 = 0.0;
-    row_gemv<double, double, K, false, true>(a.lo, s, lane, len, a.z, a0, a1, a2);
+    row_gemv<double, double, K, false, true>(a.lo, s, lane, len, a.zpos, a0, a1, a2);
     if (active && (lane & (K - 1)) == 0) {
       const int node = a.perm[row];
       const double r0 = __ldcg(&a.r[3 * node]), r1 = __ldcg(&a.r[3 * node + 1]), r2 = __ldcg(&a.r[3 * node + 2]);
       double x1 = r0 - a0, x2 = r1 - a1, x3 = r2 - a2;
       lu_solve(a.alu, a.npos, row, x1, x2, x3);
-      a.z[3 * node] = x1;
-      a.z[3 * node + 1] = x2;
-      a.z[3 * node + 2] = x3;
+      double *out = FUSE ? a.z + 3 * node : a.zpos + 3 * row;
+      out[0] = x1;
+      out[1] = x2;
+      out[2] = x3;
       if (FUSE) acc += r0 * x1 + r1 * x2 + r2 * x3;
     }
   }
@@ -195,12 +204,15 @@ __device__ __forceinline__ double team_bwd(const BatchArgs &a, const Team &t, in
     const int row = a.up.row0[s] + roff;
     const int len = active ? a.up.rowlen[s * 32 + roff] : 0;
     double x1 = 0.0, x2 = 0.0, x3 = 0.0;
-    row_gemv<double, double, K, true, true>(a.up, s, lane, len, a.z, x1, x2, x3);
+    row_gemv<double, double, K, true, true>(a.up, s, lane, len, a.zpos, x1, x2, x3);
     if (active && (lane & (K - 1)) == 0) {
       const int node = a.perm[row];
       lu_solve(a.alu, a.npos, row, x1, x2, x3);
-      const double z0 = __ldcg(&a.z[3 * node]) - x1, z1 = __ldcg(&a.z[3 * node + 1]) - x2,
-                   z2 = __ldcg(&a.z[3 * node + 2]) - x3;
+      const double z0 = __ldcg(&a.zpos[3 * row]) - x1, z1 = __ldcg(&a.zpos[3 * row + 1]) - x2,
+                   z2 = __ldcg(&a.zpos[3 * row + 2]) - x3;
+      a.zpos[3 * row] = z0;
+      a.zpos[3 * row + 1] = z1;
+      a.zpos[3 * row + 2] = z2;
       a.z[3 * node] = z0;
       a.z[3 * node + 1] = z1;
       a.z[3 * node + 2] = z2;
@@ -210,12 +222,8 @@ __device__ __forceinline__ double team_bwd(const BatchArgs &a, const Team &t, in
   return acc;
 }
 
-// The CG of one system by one team.
-template <int K>
-__device__ void team_solve(const BatchArgs &a, int id, Team &t, CgState &st, double *s_warp, double *s_red,
-                           double *s_out) {
-  const BatchSys sy = a.sys[id];
-  const int lo3 = 3 * sy.node0, n3 = 3 * sy.n;
+// The CG's scalars at the start of a solve, one replica per CTA.
+__device__ __forceinline__ void team_begin(const BatchArgs &a, CgState &st) {
   if (threadIdx.x == 0) {
     st.rho = st.rho1 = st.alpha = st.beta = st.pq = st.rr = 0.0;
     st.bnrm2 = st.resid = st.rr_true = 0.0;
@@ -231,6 +239,38 @@ __device__ void team_solve(const BatchArgs &a, int id, Team &t, CgState &st, dou
     st.rhist = nullptr;
     st.rhist_cap = st.rhist_n = 0;
   }
+}
+
+// The end of a system: its final true residual and its result.
+__device__ __forceinline__ void team_end(const BatchArgs &a, int id, Team &t, const CgState &st, double *s_warp,
+                                         double *s_red, double *s_out) {
+  const BatchSys sy = a.sys[id];
+  // final true residual ||b - A x|| / ||b|| (hecmw_rel_resid_L2_33), q as scratch
+  team_sync(t);
+  const double rt = team_sum(t, team_resid<true, false>(a, sy, t, a.x, a.q), s_warp, s_red, s_out);
+  if (t.rank == 0 && threadIdx.x == 0) {
+    BatchOut o;
+    o.iter = st.zero_rhs ? 0 : st.iter;
+    o.error = st.zero_rhs ? HECMW33_ERR_ZERO_RHS : st.error;
+    o.zero_rhs = st.zero_rhs;
+    o.resid = st.zero_rhs ? 0.0 : st.resid;
+    o.bnrm2 = st.bnrm2;
+    o.true_resid = st.bnrm2 > 0.0 ? sqrt(rt / st.bnrm2) : 0.0;
+    o.converged = st.zero_rhs || o.true_resid < st.tol;
+    o.guard = st.guard;
+    o.team = t.size;
+    a.out[id] = o;
+  }
+  team_sync(t);
+}
+
+// The CG of one system by one team.
+template <int K>
+__device__ void team_solve(const BatchArgs &a, int id, Team &t, CgState &st, double *s_warp, double *s_red,
+                           double *s_out) {
+  const BatchSys sy = a.sys[id];
+  const int lo3 = 3 * sy.node0, n3 = 3 * sy.n;
+  team_begin(a, st);
   __syncthreads();
   // prologue: r = b - A x and BNRM2 in one pass
   const double bb = team_sum(t, team_resid<false, true>(a, sy, t, a.x, a.r), s_warp, s_red, s_out);
@@ -322,29 +362,115 @@ __device__ void team_solve(const BatchArgs &a, int id, Team &t, CgState &st, dou
     __syncthreads();
     team_sync(t);  // r, x of this iteration visible before the next sweeps
   }
-  // final true residual ||b - A x|| / ||b|| (hecmw_rel_resid_L2_33), q as scratch
-  team_sync(t);
-  const double rt = team_sum(t, team_resid<true, false>(a, sy, t, a.x, a.q), s_warp, s_red, s_out);
-  if (t.rank == 0 && threadIdx.x == 0) {
-    BatchOut o;
-    o.iter = st.zero_rhs ? 0 : st.iter;
-    o.error = st.zero_rhs ? HECMW33_ERR_ZERO_RHS : st.error;
-    o.zero_rhs = st.zero_rhs;
-    o.resid = st.zero_rhs ? 0.0 : st.resid;
-    o.bnrm2 = st.bnrm2;
-    o.true_resid = st.bnrm2 > 0.0 ? sqrt(rt / st.bnrm2) : 0.0;
-    o.converged = st.zero_rhs || o.true_resid < st.tol;
-    o.guard = st.guard;
-    o.team = t.size;
-    a.out[id] = o;
+  team_end(a, id, t, st, s_warp, s_red, s_out);
+}
+
+// The fused iteration (h33_persist.cuh) of one system by one team: every vector in
+// position order (a system's positions are its node range), x back in node order at the
+// end and before every true residual.
+template <int K>
+__device__ void team_solve_fused(const BatchArgs &a, int id, Team &t, CgState &st, double *s_warp, double *s_red,
+                                 double *s_out) {
+  const BatchSys sy = a.sys[id];
+  const int lo3 = 3 * sy.node0, n3 = 3 * sy.n;
+  team_begin(a, st);
+  __syncthreads();
+  const double bb = team_sum(t, team_resid<false, true, true>(a, sy, t, a.x, a.v.r), s_warp, s_red, s_out);
+  if (threadIdx.x == 0) {
+    st.bnrm2 = bb;
+    if (bb == 0.0) {
+      st.zero_rhs = 1;
+      st.done = 1;
+    }
+    if (st.maxit <= 0) st.done = 1;
+  }
+  __syncthreads();
+  for (int i = t.tid; i < sy.n; i += t.nthreads) {
+    const int pos = sy.node0 + i, node = a.perm[pos];
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      if (st.zero_rhs) a.x[3 * node + c] = 0.0;  // hecmw_solver.f90:32-37
+      else a.px[3 * pos + c] = __ldcg(&a.x[3 * node + c]);
+      a.v.zu[3 * size_t(pos) + c] = make_double2(0.0, 0.0);
+    }
   }
   team_sync(t);
+  const auto sync = [&] { team_sync(t); };
+  const auto fwd = [&] { return GroupCursor(a.lo_desc, a.lo_gs, sy.g0, sy.g1, false, t.warp, t.nwarps); };
+  const auto nodes_x = [&] {
+    for (int i = t.tid; i < sy.n; i += t.nthreads) {
+      const int pos = sy.node0 + i, node = a.perm[pos];
+#pragma unroll
+      for (int c = 0; c < 3; c++) a.x[3 * node + c] = __ldcg(&a.px[3 * pos + c]);
+    }
+  };
+  bool restart = true;  // g from r
+  while (!st.done) {
+    if (restart) {
+      ssor_sweep<K, 2, true>(a.v, a.lo.val, a.lo.col, fwd(), sync, 0.0, false);
+      team_sync(t);
+      restart = false;
+    }
+    if (threadIdx.x == 0) st.guard++;
+    const double rho = team_sum(
+        t,
+        ssor_sweep<K, 0, true>(a.v, a.up.val, a.up.col,
+                               GroupCursor(a.up_desc, a.up_gs, sy.g0, sy.g1, true, t.warp, t.nwarps), sync, 0.0, false),
+        s_warp, s_red, s_out);
+    if (threadIdx.x == 0) fin_rho(&st, rho);
+    __syncthreads();
+    if (st.done) break;
+    const double pq = team_sum(
+        t, ssor_sweep<K, 1, true>(a.v, a.lo.val, a.lo.col, fwd(), sync, st.beta, st.iter == 1), s_warp, s_red, s_out);
+    if (threadIdx.x == 0) fin_pq(&st, pq);
+    __syncthreads();
+    if (st.done) break;
+    const bool refresh = (st.iter % kIterRecomputeR) == 0;
+    const double alpha = st.alpha;
+    double rr_part = 0.0;
+    for (int i = lo3 + t.tid; i < lo3 + n3; i += t.nthreads) {
+      a.px[i] = alpha * __ldcg(&a.v.p[i]) + __ldcg(&a.px[i]);
+      if (!refresh) {
+        const double r = -alpha * __ldcg(&a.v.q[i]) + __ldcg(&a.v.r[i]);
+        a.v.r[i] = r;
+        a.v.g[i] = -alpha * __ldcg(&a.v.h[i]) + __ldcg(&a.v.g[i]);
+        rr_part += r * r;
+      }
+    }
+    const double rr = team_sum(t, rr_part, s_warp, s_red, s_out);
+    if (!refresh) {
+      if (threadIdx.x == 0) fin_rr(&st, rr);
+      __syncthreads();
+    }
+    team_sync(t);  // x, r and g complete
+    if (refresh || st.recompute) {
+      nodes_x();
+      team_sync(t);
+      const double rt = team_sum(t, team_resid<true, false, true>(a, sy, t, a.x, a.v.r), s_warp, s_red, s_out);
+      if (threadIdx.x == 0) {
+        st.rr = rt;
+        st.resid = sqrt(rt / st.bnrm2);
+        if (st.resid <= st.tol) {
+          st.done = 1;
+          st.converged = 1;
+        }
+      }
+      team_sync(t);
+      restart = true;
+    }
+    if (threadIdx.x == 0) loop_ctl(&st, 0, 0);
+    __syncthreads();
+  }
+  if (!st.zero_rhs) nodes_x();
+  team_end(a, id, t, st, s_warp, s_red, s_out);
 }
 
 // The arguments live in device memory (written before each launch), so one captured
 // graph serves every solve of the same launch shape.
-template <int K>
-__global__ void __launch_bounds__(kThreads, 4) batch_cg_kernel(const BatchArgs *__restrict__ args) {
+// FUSED: every system by team_solve_fused, whose slices need 128 registers (two CTAs per
+// SM instead of four).
+template <int K, bool FUSED>
+__global__ void __launch_bounds__(kThreads, FUSED ? 2 : 4) batch_cg_kernel(const BatchArgs *__restrict__ args) {
   __shared__ BatchArgs a;
   __shared__ CgState st;
   __shared__ double s_warp[kWarpsPerCta];
@@ -370,7 +496,8 @@ __global__ void __launch_bounds__(kThreads, 4) batch_cg_kernel(const BatchArgs *
     const int item = *cl.map_shared_rank(&s_item, 0);
     cl.sync();  // every CTA has read the item before rank 0 draws the next one
     if (item >= a.nbig) break;
-    team_solve<K>(a, a.big[item], t, st, s_warp, s_red, &s_out);
+    if constexpr (FUSED) team_solve_fused<K>(a, a.big[item], t, st, s_warp, s_red, &s_out);
+    else team_solve<K>(a, a.big[item], t, st, s_warp, s_red, &s_out);
   }
   // phase 2: small systems, one CTA per system
   t.rank = 0;
@@ -386,7 +513,8 @@ __global__ void __launch_bounds__(kThreads, 4) batch_cg_kernel(const BatchArgs *
     const int item = s_item;
     __syncthreads();
     if (item >= a.nsmall) break;
-    team_solve<K>(a, a.small[item], t, st, s_warp, s_red, &s_out);
+    if constexpr (FUSED) team_solve_fused<K>(a, a.small[item], t, st, s_warp, s_red, &s_out);
+    else team_solve<K>(a, a.small[item], t, st, s_warp, s_red, &s_out);
   }
   // every CTA of a cluster stays until the others are done with its shared memory
   cl.sync();

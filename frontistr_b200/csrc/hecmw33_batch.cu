@@ -106,6 +106,9 @@ struct Batch {
   DevArray<BatchArgs> d_args;
   BatchArgs *h_args = nullptr;
   DevArray<double> b, x, r, z, p, q;
+  DevArray<double> zu, g, h, px;  // position order (the fused iteration; zu also the unfused sweeps' intermediate)
+  DevArray<int> iperm;
+  DevArray<int4> lo_desc, up_desc;
   // schedule and statistics
   Schedule sched;
   bool tuned = false;
@@ -243,14 +246,32 @@ void build_precond_layout(Batch &B, int lanes) {
   } else {
     reordered_rows(prof, B.perm_h, iperm, lower, upper);
   }
+  // the sweeps gather in position order
+  for (auto *br : {&lower, &upper})
+    for (int &c : br->col) c = iperm[size_t(c)];
   SellLayout lo, up;
   build_sell(lower, group_rows, lo, lanes);
   build_sell(upper, group_rows, up, lanes);
+  // padding blocks gather their own slice's first position: position 0 is another system's
+  for (auto *L : {&lo, &up})
+#pragma omp parallel for schedule(static)
+    for (int sl = 0; sl < L->nslices; sl++)
+      for (int64_t i = 32 * int64_t(L->slot0[size_t(sl)]); i < 32 * int64_t(L->slot0[size_t(sl)] + L->len[size_t(sl)]); i++)
+        if (L->src[size_t(i)] < 0) L->col[size_t(i)] = L->row0[size_t(sl)];
   B.lo.upload(lo, B.stream);
   B.up.upload(up, B.stream);
   B.lo_gs.upload(lo.group_slice, B.stream);
   B.up_gs.upload(up.group_slice, B.stream);
   B.perm.upload(B.perm_h, B.stream);
+  B.iperm.upload(iperm, B.stream);
+  auto describe = [&](const DevSellB &L, DevArray<int4> &d) {
+    d.alloc(size_t(std::max(L.nslices, 1)));
+    slice_desc_kernel<<<std::max(1, std::min((L.nslices + kThreads - 1) / kThreads, B.nsm * 8)), kThreads, 0, B.stream>>>(
+        L.slot0.p, L.len.p, L.row0.p, L.nrows.p, L.nslices, d.p);
+    H33_CUDA(cudaGetLastError());
+  };
+  describe(B.lo, B.lo_desc);
+  describe(B.up, B.up_desc);
   B.lanes_built = lanes;
   B.lo.pack(B.raw.p, B.stream, B.nsm);
   B.up.pack(B.raw.p, B.stream, B.nsm);
@@ -262,6 +283,31 @@ void build_precond_layout(Batch &B, int lanes) {
   B.sys_d.upload(B.sys_h, B.stream);
   B.drop_graph();
   B.sync();
+}
+
+// The schedule before any tuning: every system to a team of C CTAs, C by the larger of
+// the largest system's time on its team and the whole batch's over the resident teams,
+// with a system's time as nodes / C + 230 (the part that more CTAs do not shorten, in
+// nodes); four lanes per row where the systems are large.  Measured with 8 lanes and
+// C = 1 / 2 / 4 / 8 (ms a solve): 64 systems of 4-20 elements an edge 153 / 89 / 48.8 /
+// 34.4, 6 of 4-14 29.8 / 20.4 / 15.3 / 11.5, 128 of 4-14 42.4 / 28.5 / 21.9 / 36.3, 100 of
+// 12-24 422 / 227 / 133 / 128 (four lanes: C = 4 105, C = 8 115); the fixed choice before,
+// teams of 4 for the largest 15 %, took 72.6, 22.8, 23.9 and 250.
+Schedule default_schedule(const Batch &B) {
+  const double slots = 2.0 * B.nsm, mean = double(B.N) / B.nsys;
+  double largest = 0.0, best = 0.0;
+  for (int s = 0; s < B.nsys; s++) largest = std::max(largest, double(B.node0[size_t(s) + 1] - B.node0[size_t(s)]));
+  Schedule sc;
+  for (int c : {1, 2, 4, 8}) {
+    const double cost = std::max(largest / c + 230.0, B.nsys * c / slots * (mean / c + 230.0));
+    if (c == 1 || cost < best) {
+      best = cost;
+      sc.cluster = c;
+    }
+  }
+  sc.lanes = mean > 4096.0 ? 4 : 8;
+  sc.big_frac = sc.cluster > 1 ? 1.0 : 0.0;
+  return sc;
 }
 
 void batch_set_matrix(Batch &B, int nsys, const int *sys_ptr, int N, int NP, int NPL, int NPU, const int *indexL,
@@ -326,6 +372,9 @@ void batch_set_matrix(Batch &B, int nsys, const int *sys_ptr, int N, int NP, int
     }
     const size_t n3 = size_t(3) * N;
     for (auto *v : {&B.b, &B.x, &B.r, &B.z, &B.p, &B.q}) v->alloc(n3);
+    B.zu.alloc(2 * n3);
+    if (kind == 1)
+      for (auto *v : {&B.g, &B.h, &B.px}) v->alloc(n3);
     B.out.alloc(size_t(nsys));
     if (B.h_out) cudaFreeHost(B.h_out);
     B.h_out = nullptr;
@@ -348,6 +397,7 @@ void batch_set_matrix(Batch &B, int nsys, const int *sys_ptr, int N, int NP, int
       for (int j = 0; j < 3; j++)
         if (std::fabs(D[9 * size_t(i) + 4 * j]) == 0.0) B.zero_diag[s] = 1;
   if (symbolic) {
+    if (!B.tuned) B.sched = default_schedule(B);
     build_precond_layout(B, B.sched.lanes);
   } else {
     // values only: repack the sweep layouts and refactor the diagonal blocks
@@ -432,39 +482,30 @@ cudaLaunchConfig_t launch_config(Batch &B, int cluster, int grid, cudaLaunchAttr
   return cfg;
 }
 
-template <int K>
-void launch_batch_k(Batch &B, const BatchArgs *a, int cluster, int grid) {
+// Calls f with the kernel for the built layouts (the fused one needs four lanes per row).
+template <class F>
+auto with_kernel(const Batch &B, bool fused, F f) {
+  switch (B.lanes_built) {
+    case 2: return f(batch_cg_kernel<2, false>);
+    case 4: return f(fused ? batch_cg_kernel<4, true> : batch_cg_kernel<4, false>);
+    case 16: return f(fused ? batch_cg_kernel<16, true> : batch_cg_kernel<16, false>);
+    default: return f(fused ? batch_cg_kernel<8, true> : batch_cg_kernel<8, false>);
+  }
+}
+
+void launch_batch(Batch &B, bool fused, const BatchArgs *a, int cluster, int grid) {
   cudaLaunchAttribute attr[1];
   cudaLaunchConfig_t cfg = launch_config(B, cluster, grid, attr);
-  H33_CUDA(cudaLaunchKernelEx(&cfg, batch_cg_kernel<K>, a));
+  with_kernel(B, fused, [&](auto kern) { H33_CUDA(cudaLaunchKernelEx(&cfg, kern, a)); });
 }
 
 // CTAs of the persistent grid: as many clusters as can be resident at once.
-template <int K>
-int resident_grid(Batch &B, int cluster) {
+int batch_grid(Batch &B, bool fused, int cluster) {
   cudaLaunchAttribute attr[1];
   cudaLaunchConfig_t cfg = launch_config(B, cluster, cluster * B.nsm, attr);
   int ncl = 0;
-  H33_CUDA(cudaOccupancyMaxActiveClusters(&ncl, batch_cg_kernel<K>, &cfg));
+  with_kernel(B, fused, [&](auto kern) { H33_CUDA(cudaOccupancyMaxActiveClusters(&ncl, kern, &cfg)); });
   return std::max(1, ncl) * cluster;
-}
-
-void launch_batch(Batch &B, const BatchArgs *a, int cluster, int grid) {
-  switch (B.lanes_built) {
-    case 2: return launch_batch_k<2>(B, a, cluster, grid);
-    case 4: return launch_batch_k<4>(B, a, cluster, grid);
-    case 16: return launch_batch_k<16>(B, a, cluster, grid);
-    default: return launch_batch_k<8>(B, a, cluster, grid);
-  }
-}
-
-int batch_grid(Batch &B, int cluster) {
-  switch (B.lanes_built) {
-    case 2: return resident_grid<2>(B, cluster);
-    case 4: return resident_grid<4>(B, cluster);
-    case 16: return resident_grid<16>(B, cluster);
-    default: return resident_grid<8>(B, cluster);
-  }
 }
 
 // Queues for this solve: systems by decreasing estimated work (blocks x expected
@@ -499,7 +540,9 @@ float run_batch(Batch &B, const Schedule &sc, int iterpremax, double tol, int ma
   for (int s = 0; s < B.nsys; s++) B.sys_h[s].skip = (B.zero_diag[s] && iterpremax > 0) ? 1 : 0;
   B.sys_d.upload(B.sys_h, B.stream);
   make_queues(B, sc);
-  const int grid = batch_grid(B, sc.cluster);
+  // the sweeps hold A's own values in a batch: matrix and preconditioner change together
+  const bool fused = B.kind == 1 && iterpremax == 1 && B.sigma == 1.0 && B.lanes_built >= 4;
+  const int grid = batch_grid(B, fused, sc.cluster);
   BatchArgs a;
   a.A = B.A.view();
   a.lo = B.lo.view();
@@ -523,6 +566,12 @@ float run_batch(Batch &B, const Schedule &sc, int iterpremax, double tol, int ma
   a.z = B.z.p;
   a.p = B.p.p;
   a.q = B.q.p;
+  a.lo_desc = B.lo_desc.p;
+  a.up_desc = B.up_desc.p;
+  a.iperm = B.iperm.p;
+  a.zpos = B.zu.p;
+  a.px = B.px.p;
+  a.v = SsorVecs{B.alu.p, B.N, B.r.p, B.g.p, B.p.p, B.q.p, B.h.p, reinterpret_cast<double2 *>(B.zu.p)};
   a.out = B.out.p;
   a.tol = tol;
   a.maxit = maxit;
@@ -530,12 +579,12 @@ float run_batch(Batch &B, const Schedule &sc, int iterpremax, double tol, int ma
   H33_CUDA(cudaMemcpyAsync(B.d_args.p, B.h_args, sizeof(BatchArgs), cudaMemcpyHostToDevice, B.stream));
   // the solve as one graph: queue reset + the persistent kernel (its arguments are
   // read from d_args, so the graph depends only on the launch shape)
-  const int key[4] = {sc.lanes, sc.cluster, grid, 0};
+  const int key[4] = {sc.lanes, sc.cluster, grid, fused ? 1 : 0};
   if (!(B.exec && std::equal(key, key + 4, B.gkey))) {
     B.drop_graph();
     H33_CUDA(cudaStreamBeginCapture(B.stream, cudaStreamCaptureModeThreadLocal));
     H33_CUDA(cudaMemsetAsync(B.queue.p, 0, 2 * sizeof(int), B.stream));
-    launch_batch(B, B.d_args.p, sc.cluster, grid);
+    launch_batch(B, fused, B.d_args.p, sc.cluster, grid);
     H33_CUDA(cudaStreamEndCapture(B.stream, &B.graph));
     H33_CUDA(cudaGraphInstantiate(&B.exec, B.graph, 0));
     std::copy(key, key + 4, B.gkey);

@@ -160,3 +160,50 @@ def test_batch_autotune_and_cache(batch12, tmp_path, monkeypatch):
         info2 = bs.info()
     assert info2["tuned"] == 1 and (info2["lanes"], info2["cluster"]) == (info["lanes"], info["cluster"])
     check_against_oracle(systems, sys_ptr, X, rec, refs)
+
+
+@pytest.mark.parametrize("schedule", [None, "2,4,1", "8,4,1"])
+@pytest.mark.parametrize("sigma", [1.0, 1.2])
+def test_batch_fused_and_unfused_iterations(schedule, sigma, monkeypatch):
+    """The fused iteration (SIGMA_DIAG = 1, four lanes per row or more) and the sweeps
+    with a product beside them, under the untuned schedule and fixed ones."""
+    if schedule is None:
+        monkeypatch.delenv("HECMW33_BATCH_SCHEDULE", raising=False)
+        monkeypatch.setenv("HECMW33_AUTOTUNE_CACHE", "/nonexistent/tune.jsonl")
+    else:
+        monkeypatch.setenv("HECMW33_BATCH_SCHEDULE", schedule)
+    systems = random_box_batch(7, edge_range=(1, 9), seed=21)
+    refs = []
+    for m in systems:
+        mm = m.copy()
+        mm.set_sigma_diag(sigma)
+        mm.set_iter(20000)
+        refs.append(Oracle(mm).solve(coloured=1))
+    big, sys_ptr = stack_systems(systems)
+    ia, ra = flags(big)
+    ra[1] = sigma
+    X = np.zeros(3 * big.N)
+    with BatchSolver() as bs:
+        bs.set_matrix(big, sys_ptr, ia, ra)
+        rec = bs.solve(big.B, X, ia, ra)
+    check_against_oracle(systems, sys_ptr, X, rec, refs)
+
+
+def test_batch_system_that_diverges_leaves_the_others_alone(monkeypatch):
+    """Not-a-numbers of one system (the first: padding blocks must not gather from it)."""
+    monkeypatch.setenv("HECMW33_BATCH_SCHEDULE", "8,2,1")
+    systems = random_box_batch(4, edge_range=(2, 6), seed=9)
+    refs = oracle_solutions(systems)
+    bad = systems[0].copy()
+    bad.D[:] = np.nan
+    big, sys_ptr = stack_systems([bad] + systems[1:])
+    ia, ra = flags(big)
+    X = np.zeros(3 * big.N)
+    with BatchSolver() as bs:
+        bs.set_matrix(big, sys_ptr, ia, ra)
+        rec = bs.solve(big.B, X, ia, ra)
+    assert rec["errors"][0] == 3004
+    for k in (1, 2, 3):
+        x = X[3 * sys_ptr[k]:3 * sys_ptr[k + 1]]
+        assert rec["errors"][k] == 0 and abs(int(rec["iter"][k]) - refs[k]["iter"]) <= 2
+        assert np.linalg.norm(x - refs[k]["X"]) <= 1e-8 * np.linalg.norm(refs[k]["X"])
