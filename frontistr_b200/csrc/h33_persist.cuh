@@ -115,44 +115,38 @@ struct PersistShared {
   int dead;
 };
 
-// Every write made before persist_arrive by any CTA is visible after persist_wait.
-// CLUSTER: the grid is one cluster and the barrier its hardware barrier; else a counter
-// in global memory, its wait bounded.
+// One thread's wait until *bar has reached target; after kPSpin polls, or when another
+// CTA has given up, it gives up (dead).
+__device__ __forceinline__ void grid_wait(unsigned *bar, unsigned target, int &dead) {
+  unsigned v;
+  int tries = 0;
+  for (;;) {
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
+    if (int(v - target) >= 0) break;
+    if (dead || ++tries > kPSpin || ((tries & 1023) == 0 && *((volatile unsigned *)(bar + 1)))) {
+      dead = 1;
+      *((volatile unsigned *)(bar + 1)) = 1u;
+      break;
+    }
+  }
+}
+
+// Every write made before it by any CTA is visible after it.  CLUSTER: the grid is one
+// cluster and the barrier its hardware barrier; else a counter in global memory, its
+// wait bounded.
 template <bool CLUSTER>
-__device__ __forceinline__ void persist_arrive(const PersistArgs &a, unsigned &target) {
+__device__ __forceinline__ void persist_barrier(const PersistArgs &a, PersistShared &sh, unsigned &target) {
   if constexpr (CLUSTER) {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
   } else {
     target += gridDim.x;
     __syncthreads();
-    if (threadIdx.x == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.bar) : "memory");
-  }
-}
-template <bool CLUSTER>
-__device__ __forceinline__ void persist_wait(const PersistArgs &a, PersistShared &sh, unsigned target) {
-  if constexpr (CLUSTER) {
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-  } else {
     if (threadIdx.x == 0) {
-      unsigned v;
-      int tries = 0;
-      for (;;) {
-        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(a.bar) : "memory");
-        if (int(v - target) >= 0) break;
-        if (sh.dead || ++tries > kPSpin || ((tries & 1023) == 0 && *((volatile unsigned *)(a.bar + 1)))) {
-          sh.dead = 1;
-          *((volatile unsigned *)(a.bar + 1)) = 1u;
-          break;
-        }
-      }
+      asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.bar) : "memory");
+      grid_wait(a.bar, target, sh.dead);
     }
     __syncthreads();
   }
-}
-template <bool CLUSTER>
-__device__ __forceinline__ void persist_barrier(const PersistArgs &a, PersistShared &sh, unsigned &target) {
-  persist_arrive<CLUSTER>(a, target);
-  persist_wait<CLUSTER>(a, sh, target);
 }
 
 // Sum over the grid, the same value in every thread; includes a barrier.
