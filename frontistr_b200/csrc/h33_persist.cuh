@@ -607,6 +607,110 @@ __global__ void __launch_bounds__(32 * persist_warps<K>(), 1) cg_ssor_persist_ke
   if constexpr (CLUSTER) persist_barrier<true>(a, sh, target);
 }
 
+// ---- one application of the SSOR ---------------------------------------------------
+// z = M^-1 r in one launch, for the methods whose loop is not one (BiCGSTAB, GMRES, ...):
+// the colour kernels' arithmetic in their order (sweep_fwd_uni_kernel,
+// sweep_bwd_uni_kernel), a grid barrier where they have a launch.  bar: arrivals, whether
+// a wait gave up, CTAs that are done (the last sets the first and third back to zero).
+struct ApplyArgs {
+  SellView<double> lo, up;
+  const int4 *lo_items, *up_items;
+  int lo_stride, up_stride;
+  const int *perm;
+  const double *alu;
+  int n, ncolor;
+  const double *r;
+  double *z, *zpos;
+  const CgState *st;
+  unsigned *bar;
+};
+
+template <int K>
+__global__ void __launch_bounds__(32 * persist_warps<K>(), 1) ssor_apply_persist_kernel(const ApplyArgs a) {
+  if (a.st && a.st->done) return;
+  __shared__ int dead;
+  const int lane = threadIdx.x & 31, roff = lane / K;
+  const bool leader = (lane & (K - 1)) == 0;
+  const int w = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+  unsigned target = 0;
+  if (threadIdx.x == 0) dead = 0;
+  const auto barrier = [&] {
+    target += gridDim.x;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.bar) : "memory");
+      grid_wait(a.bar, target, dead);
+    }
+    __syncthreads();
+  };
+  {
+    ListCursor cur{a.lo_items + size_t(w) * a.lo_stride, a.ncolor};
+    int4 it = cur.next();
+    for (int c = 0; c < a.ncolor; c++) {
+      if (c) barrier();
+      while ((it.w >> 6) == c) {
+        const int row = it.z + roff;
+        const bool act = roff < (it.w & 63) && leader;
+        double r0 = 0.0, r1 = 0.0, r2 = 0.0;
+        if (act) {
+          const int node = a.perm[row];
+          r0 = a.r[3 * node];
+          r1 = a.r[3 * node + 1];
+          r2 = a.r[3 * node + 2];
+        }
+        double y0 = 0.0, y1 = 0.0, y2 = 0.0;
+        slice_gemv_u<double, double, K, false, true>(a.lo, it.x, it.y, lane, a.zpos, y0, y1, y2);
+        if (act) {
+          double x1 = r0 - y0, x2 = r1 - y1, x3 = r2 - y2;
+          lu_solve(a.alu, a.n, row, x1, x2, x3);
+          a.zpos[3 * row] = x1;
+          a.zpos[3 * row + 1] = x2;
+          a.zpos[3 * row + 2] = x3;
+        }
+        it = cur.next();
+      }
+    }
+  }
+  ListCursor cur{a.up_items + size_t(w) * a.up_stride, a.ncolor};
+  int4 it = cur.next();
+  for (int c = 0; c < a.ncolor; c++) {
+    barrier();
+    while ((it.w >> 6) == c) {
+      const int row = it.z + roff;
+      const bool act = roff < (it.w & 63) && leader;
+      int node = 0;
+      double c0 = 0.0, c1 = 0.0, c2 = 0.0;
+      if (act) {
+        node = a.perm[row];
+        c0 = __ldcg(a.zpos + 3 * row);
+        c1 = __ldcg(a.zpos + 3 * row + 1);
+        c2 = __ldcg(a.zpos + 3 * row + 2);
+      }
+      double x1 = 0.0, x2 = 0.0, x3 = 0.0;
+      slice_gemv_u<double, double, K, true, true>(a.up, it.x, it.y, lane, a.zpos, x1, x2, x3);
+      if (act) {
+        lu_solve(a.alu, a.n, row, x1, x2, x3);
+        const double z0 = c0 - x1, z1 = c1 - x2, z2 = c2 - x3;
+        a.zpos[3 * row] = z0;
+        a.zpos[3 * row + 1] = z1;
+        a.zpos[3 * row + 2] = z2;
+        a.z[3 * node] = z0;
+        a.z[3 * node + 1] = z1;
+        a.z[3 * node + 2] = z2;
+      }
+      it = cur.next();
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(a.bar + 2, 1u) == gridDim.x - 1) {
+      a.bar[0] = 0u;
+      a.bar[2] = 0u;
+    }
+  }
+}
+
 // ---- block ILU ----------------------------------------------------------------------
 // The CG with a block ILU(p) preconditioner, whose levels take the place of the colours:
 // its triangles are not A's, so q = A p is a pass of its own, and the vectors stay in

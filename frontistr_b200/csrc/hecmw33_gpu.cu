@@ -451,6 +451,7 @@ struct Solver {
   Precond pc;
   PersistPlan pp;
   MrPersistPlan mpp;
+  bool apply_one = false;  // this solve applies its SSOR in one launch (apply_rule)
   // FP32 copies for the mixed-precision refinement
   DevArray<float> bf, xf, rf, zf, pf, qf, wf, zpf;
   // flexible CG buffers (SSOR output and previous residual) and the learned preconditioner
@@ -1398,10 +1399,40 @@ void launch_sweep_t(Solver &S, const Precond &P, const SellView<TV> &lo, const S
   }
 }
 
+// Whether one application of the solve's SSOR runs as ssor_apply_persist_kernel: up to
+// 17,760 rows a colour on 148 SMs, as far as it was measured.  BiCGSTAB, us an iteration as
+// colour launches / in one launch per application: 0.7 thousand nodes 299 / 238, 20
+// thousand 561 / 371, 36 thousand 612 / 382, 118 thousand (7,350 rows a colour) 675 / 456,
+// 275 thousand (17 thousand rows) 863 / 822; GMRES(30) on 20 thousand 494 / 371.  persist_plan<4> has to have run.
+bool apply_rule(const Solver &S) {
+  const Precond &P = S.pc;
+  return P.valid && P.kind == 1 && P.pos_cols && P.lo.lanes == 4 && S.N / std::max(P.ncolor, 1) <= 120 * S.nsm;
+}
+
+void launch_apply_persist(Solver &S, const double *rin, double *zout, double *zpos, const CgState *st) {
+  const Precond &P = S.pc;
+  const PersistPlan &L = S.pp;
+  ApplyArgs a{P.lo.view(), P.up.view(), L.lo_items.p, L.up_items.p, L.lo_stride, L.up_stride, P.perm_fwd.p,
+              P.alu_fwd.p, S.N, int(P.lo.group_slice.size()) - 1, rin, zout, zpos, st, L.bar.p + 4};
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(unsigned(L.grid), 1, 1);
+  cfg.blockDim = dim3(32 * persist_warps<4>(), 1, 1);
+  cfg.stream = S.stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  H33_CUDA(cudaLaunchKernelEx(&cfg, ssor_apply_persist_kernel<4>, a));
+}
+
 // dpos (may be null; multicolour layouts only): the backward sweep's correction y - z
 // per colour position, for lower_resid_kernel.
 template <class R, bool FUSE_RHO>
 void launch_sweep(Solver &S, const Views<R> &V, const R *rin, R *zout, CgState *st, R *dpos = nullptr) {
+  if constexpr (!FUSE_RHO && std::is_same<R, double>::value) {
+    if (S.apply_one && V.pc == &S.pc && !V.lowp && !dpos) return launch_apply_persist(S, rin, zout, V.zpos, st);
+  }
   if (V.lowp)
     launch_sweep_t<R, __nv_bfloat16, float, FUSE_RHO>(S, *V.pc, V.lo16, V.up16, V.alu32_f, V.alu32_b, rin, zout,
                                                       V.zpos, st, dpos);
@@ -1703,7 +1734,7 @@ void build_graph(Solver &S, int iterpremax, int mode = 0) {
   const int flexible = mode & 1;
   const int lowp = (mode & 4) ? 1 : 0;
   const int key[5] = {S.generation, S.pc.generation, S.pc.kind, iterpremax,
-                      mode + (flexible ? S.L.graph_generation * 4 : 0)};
+                      mode + (flexible ? S.L.graph_generation * 4 : 0) + (S.apply_one ? 1 << 24 : 0)};
   if (G.exec && std::equal(key, key + 5, G.key)) return;
   G.drop();
   const Views<R> V = views(S, R(), lowp, flexible ? &S.L.sm : nullptr);
@@ -1904,7 +1935,8 @@ void persist_plan(Solver &S) {
     L.zu.alloc(6 * size_t(S.N));
   }
   L.parts.alloc(3 * size_t(L.grid));
-  L.bar.alloc(2);
+  L.bar.alloc(8);  // [0, 1] the CG's, [4, 6] the single application's
+  L.bar.zero(S.stream);
   L.generation = P.generation;
 }
 
@@ -3615,6 +3647,12 @@ int solve_fp64(Solver &S, int *Iarray, double *Rarray, int *iter, double *resid,
     if (learned) ensure_lowp(S, S.L.sm);
     else ensure_lowp(S);
   }
+  S.apply_one = !persist() && !learned && !record && method != 1 && !lowp && iterPREmax > 0 && apply_rule(S);
+  if (S.apply_one) persist_plan<4>(S);
+  struct ApplyScope {
+    Solver &S;
+    ~ApplyScope() { S.apply_one = false; }
+  } apply_scope{S};
   setup_mark("solve: BF16 copies, buffers");
   if (graph_mode() && !record && !persist() && (method == 1 || method == 2))
     build_graph<double>(S, iterPREmax, learned | (lowp ? 4 : 0) | (method == 2 ? 8 : 0));
@@ -3683,6 +3721,15 @@ int solve_fp64(Solver &S, int *Iarray, double *Rarray, int *iter, double *resid,
   if (scaling.on) {
     scaling.restore();
     S.bnrm2 = dot_device(S, S.b.p, S.b.p);
+  }
+  if (S.apply_one) {
+    unsigned gave_up = 0;
+    H33_CUDA(cudaMemcpyAsync(&gave_up, S.pp.bar.p + 5, sizeof(unsigned), cudaMemcpyDeviceToHost, S.stream));
+    S.sync();
+    if (gave_up) {
+      S.pp.bar.zero(S.stream);
+      throw Failure(HECMW33_ERR_TIMEOUT, "a wait of the SSOR application gave up (internal error)");
+    }
   }
   const double resid2 = rel_resid_device(S);
   if (resid2 < TOL) Iarray[80] = 1;
