@@ -9,8 +9,8 @@
 //      preconditioner recycle policy (hecmw_matrix_misc.F90:858-877).
 //   3. preconditioner setup per flags 97/98: SSOR (RCM + multicolour ordering,
 //      reordered L/U in colour order, diagonal LU), DIAG, or block ILU(0).
-//   4. the whole CG loop (hecmw_solver_CG.f90:164-279) runs as ONE CUDA graph launch:
-//      a prologue (r = b - A x0, ||b||^2) and a conditional WHILE node whose body is one
+//   4. the whole CG loop (hecmw_solver_CG.f90:164-279) runs as ONE launch: a persistent
+//      kernel (h33_persist.cuh) for SSOR and block ILU, else a CUDA graph with a prologue (r = b - A x0, ||b||^2) and a conditional WHILE node whose body is one
 //      iteration; the device decides when the loop ends (cudaGraphSetConditional).
 //   5. true relative residual and the converged/diverged flags (Iterative.f90:131-157).
 #include <cuda_runtime.h>
@@ -1403,7 +1403,8 @@ void launch_sweep_t(Solver &S, const Precond &P, const SellView<TV> &lo, const S
 // 17,760 rows a colour on 148 SMs, as far as it was measured.  BiCGSTAB, us an iteration as
 // colour launches / in one launch per application: 0.7 thousand nodes 299 / 238, 20
 // thousand 561 / 371, 36 thousand 612 / 382, 118 thousand (7,350 rows a colour) 675 / 456,
-// 275 thousand (17 thousand rows) 863 / 822; GMRES(30) on 20 thousand 494 / 371.  persist_plan<4> has to have run.
+// 275 thousand (17 thousand rows) 863 / 822; GMRES(30) on 20 thousand 494 / 371.
+// persist_plan<4> has to have run.
 bool apply_rule(const Solver &S) {
   const Precond &P = S.pc;
   return P.valid && P.kind == 1 && P.pos_cols && P.lo.lanes == 4 && S.N / std::max(P.ncolor, 1) <= 120 * S.nsm;
