@@ -37,6 +37,7 @@ struct MrPersistArgs {
   const CgParams *prm;
   double *parts;               // 3 x gridDim.x x 16
   unsigned *bar;
+  int polls;
   int n, ncolor, nrhs;
 };
 
@@ -52,10 +53,7 @@ struct MrShared {
 __device__ __forceinline__ void mr_persist_barrier(const MrPersistArgs &a, MrShared &sh, unsigned &target) {
   target += gridDim.x;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.bar) : "memory");
-    grid_wait(a.bar, target, sh.dead);
-  }
+  if (threadIdx.x == 0) grid_meet(a.bar, target, a.polls, sh.dead);
   __syncthreads();
 }
 
@@ -364,7 +362,7 @@ __global__ void __launch_bounds__(kMrThreads, 1) mr_cg_persist_kernel(const MrPe
       a.ctl->all_done = 1;
       a.ctl->guard = guard;
       a.ctl->nrhs = a.nrhs;
-      a.ctl->fault = sh.dead;
+      a.ctl->fault = 0;  // a barrier that gave up: bar[1], read by the host
       for (int i = 0; i < 8; i++) a.ctl->ticket[i] = 0u;  // the kernels after this one count from zero
     }
   }

@@ -48,7 +48,6 @@ constexpr int persist_warps() {
   return K >= 8 ? 12 : 16;
 }
 constexpr int kPEnd = 0x7fffffff;            // end of a warp's list
-constexpr int kPSpin = 1 << 23;              // polls of a grid barrier before it gives up (seconds)
 
 // One sweep direction: the blocks and, for each warp of the grid, its slices in the
 // order of the sweep: (first slot, slots, first row, step << 6 | rows), kPEnd in w ends it.
@@ -83,7 +82,8 @@ struct PersistArgs {
   CgState *st;
   const CgParams *prm;
   double *parts;            // 3 x gridDim.x partial sums
-  unsigned *bar;            // [0] arrivals at the grid barrier, [1] set when a wait gave up
+  unsigned *bar;            // [0] arrivals at the grid barrier, [1] set when a wait gave up (the host reads it)
+  int polls;                // of a grid barrier before it gives up
   int n, ncolor;
 };
 
@@ -115,15 +115,19 @@ struct PersistShared {
   int dead;
 };
 
-// One thread's wait until *bar has reached target; after kPSpin polls, or when another
-// CTA has given up, it gives up (dead).
-__device__ __forceinline__ void grid_wait(unsigned *bar, unsigned target, int &dead) {
+// One thread's arrival at the grid barrier and its wait until *bar has reached target;
+// after `polls` polls, or when another CTA has given up, it gives up (dead).  A CTA that
+// has given up arrives nowhere any more, so none passes a barrier that a late one has not
+// reached; the others see its mark in bar[1] and give up too.
+__device__ __forceinline__ void grid_meet(unsigned *bar, unsigned target, int polls, int &dead) {
+  if (dead) return;
+  asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
   unsigned v;
   int tries = 0;
   for (;;) {
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
     if (int(v - target) >= 0) break;
-    if (dead || ++tries > kPSpin || ((tries & 1023) == 0 && *((volatile unsigned *)(bar + 1)))) {
+    if (++tries > polls || ((tries & 1023) == 0 && *((volatile unsigned *)(bar + 1)))) {
       dead = 1;
       *((volatile unsigned *)(bar + 1)) = 1u;
       break;
@@ -141,10 +145,7 @@ __device__ __forceinline__ void persist_barrier(const PersistArgs &a, PersistSha
   } else {
     target += gridDim.x;
     __syncthreads();
-    if (threadIdx.x == 0) {
-      asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.bar) : "memory");
-      grid_wait(a.bar, target, sh.dead);
-    }
+    if (threadIdx.x == 0) grid_meet(a.bar, target, a.polls, sh.dead);
     __syncthreads();
   }
 }
@@ -623,6 +624,7 @@ struct ApplyArgs {
   double *z, *zpos;
   const CgState *st;
   unsigned *bar;
+  int polls;
 };
 
 template <int K>
@@ -637,10 +639,7 @@ __global__ void __launch_bounds__(32 * persist_warps<K>(), 1) ssor_apply_persist
   const auto barrier = [&] {
     target += gridDim.x;
     __syncthreads();
-    if (threadIdx.x == 0) {
-      asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.bar) : "memory");
-      grid_wait(a.bar, target, dead);
-    }
+    if (threadIdx.x == 0) grid_meet(a.bar, target, a.polls, dead);
     __syncthreads();
   };
   {

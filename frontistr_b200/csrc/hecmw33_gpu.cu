@@ -184,6 +184,13 @@ int ssor_lanes(int n, int ncolor, int nsm) {
   return rows <= 24 * nsm ? 8 : 4;
 }
 
+// Polls of a one-launch solve's grid barrier before it gives up with error 9103: some five
+// seconds, far above any wait between CTAs that are all resident.
+int barrier_polls() {
+  const char *e = std::getenv("HECMW33_BARRIER_POLLS");
+  return e ? std::max(1, std::atoi(e)) : 1 << 23;
+}
+
 double wall() {
   return std::chrono::duration<double>(std::chrono::steady_clock::now().time_since_epoch()).count();
 }
@@ -447,6 +454,7 @@ struct Solver {
   DevArray<CgParams> params;
   CgParams *h_params = nullptr;
   CgState *h_state = nullptr;
+  unsigned *h_gave_up = nullptr;  // a one-launch solve's mark that a barrier gave up
   DevArray<int> d_err;
   Precond pc;
   PersistPlan pp;
@@ -560,6 +568,7 @@ struct Solver {
     H33_CUDA(cudaMallocHost(&h_params, sizeof(CgParams)));
     std::memset(h_params, 0, sizeof(CgParams));
     H33_CUDA(cudaMallocHost(&h_state, sizeof(CgState)));
+    H33_CUDA(cudaMallocHost(&h_gave_up, sizeof(unsigned)));
     H33_CUDA(cudaMallocHost(&h_mst, sizeof(CgState) * kMaxRhs));
     H33_CUDA(cudaMallocHost(&h_mctl, sizeof(MultiCtl)));
     state.alloc(1);
@@ -574,6 +583,7 @@ struct Solver {
     if (ev1) cudaEventDestroy(ev1);
     if (h_params) cudaFreeHost(h_params);
     if (h_state) cudaFreeHost(h_state);
+    if (h_gave_up) cudaFreeHost(h_gave_up);
     if (h_mst) cudaFreeHost(h_mst);
     if (h_mctl) cudaFreeHost(h_mctl);
     if (stream) {
@@ -1414,7 +1424,7 @@ void launch_apply_persist(Solver &S, const double *rin, double *zout, double *zp
   const Precond &P = S.pc;
   const PersistPlan &L = S.pp;
   ApplyArgs a{P.lo.view(), P.up.view(), L.lo_items.p, L.up_items.p, L.lo_stride, L.up_stride, P.perm_fwd.p,
-              P.alu_fwd.p, S.N, int(P.lo.group_slice.size()) - 1, rin, zout, zpos, st, L.bar.p + 4};
+              P.alu_fwd.p, S.N, int(P.lo.group_slice.size()) - 1, rin, zout, zpos, st, L.bar.p + 4, barrier_polls()};
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(unsigned(L.grid), 1, 1);
   cfg.blockDim = dim3(32 * persist_warps<4>(), 1, 1);
@@ -2005,6 +2015,7 @@ float run_cg_persist(Solver &S, double tol, int maxit, int *kernels) {
   a.prm = S.params.p;
   a.parts = L.parts.p;
   a.bar = L.bar.p;
+  a.polls = barrier_polls();
   a.n = S.N;
   a.ncolor = int(P.lo.group_slice.size()) - 1;
   H33_CUDA(cudaMemcpyAsync(S.params.p, S.h_params, sizeof(CgParams), cudaMemcpyHostToDevice, S.stream));
@@ -2017,11 +2028,13 @@ float run_cg_persist(Solver &S, double tol, int maxit, int *kernels) {
   }
   H33_CUDA(cudaEventRecord(S.ev1, S.stream));
   H33_CUDA(cudaMemcpyAsync(S.h_state, S.state.p, sizeof(CgState), cudaMemcpyDeviceToHost, S.stream));
+  // whichever CTA gave up: the one that writes the state may have passed every barrier
+  H33_CUDA(cudaMemcpyAsync(S.h_gave_up, L.bar.p + 1, sizeof(unsigned), cudaMemcpyDeviceToHost, S.stream));
   S.sync();
   if (kernels) *kernels += 1;
   float ms = 0.0f;
   H33_CUDA(cudaEventElapsedTime(&ms, S.ev0, S.ev1));
-  if (S.h_state->error == HECMW33_ERR_TIMEOUT)
+  if (*S.h_gave_up || S.h_state->error == HECMW33_ERR_TIMEOUT)
     throw Failure(HECMW33_ERR_TIMEOUT, "a wait of the persistent CG gave up (internal error)");
   return ms;
 }
@@ -3724,10 +3737,9 @@ int solve_fp64(Solver &S, int *Iarray, double *Rarray, int *iter, double *resid,
     S.bnrm2 = dot_device(S, S.b.p, S.b.p);
   }
   if (S.apply_one) {
-    unsigned gave_up = 0;
-    H33_CUDA(cudaMemcpyAsync(&gave_up, S.pp.bar.p + 5, sizeof(unsigned), cudaMemcpyDeviceToHost, S.stream));
+    H33_CUDA(cudaMemcpyAsync(S.h_gave_up, S.pp.bar.p + 5, sizeof(unsigned), cudaMemcpyDeviceToHost, S.stream));
     S.sync();
-    if (gave_up) {
+    if (*S.h_gave_up) {
       S.pp.bar.zero(S.stream);
       throw Failure(HECMW33_ERR_TIMEOUT, "a wait of the SSOR application gave up (internal error)");
     }
@@ -4266,6 +4278,7 @@ void run_mr_persist(Solver &S, int nrhs) {
   a.prm = S.params.p;
   a.parts = L.parts.p;
   a.bar = L.bar.p;
+  a.polls = barrier_polls();
   a.n = S.N;
   a.ncolor = int(P.lo.group_slice.size()) - 1;
   a.nrhs = nrhs;
@@ -4336,9 +4349,12 @@ float run_multi_chunk(Solver &S, int nrhs, const double *dB, double *dX, int ite
   H33_CUDA(cudaGetLastError());
   H33_CUDA(cudaMemcpyAsync(S.h_mst, S.mst.p, sizeof(CgState) * kMaxRhs, cudaMemcpyDeviceToHost, s));
   H33_CUDA(cudaMemcpyAsync(S.h_mctl, S.mctl.p, sizeof(MultiCtl), cudaMemcpyDeviceToHost, s));
+  if (persist) H33_CUDA(cudaMemcpyAsync(S.h_gave_up, S.mpp.bar.p + 1, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
   S.sync();
   float ms = 0.0f;
   H33_CUDA(cudaEventElapsedTime(&ms, S.ev0, S.ev1));
+  if (persist && *S.h_gave_up)
+    throw Failure(HECMW33_ERR_TIMEOUT, "a wait of the persistent multi-RHS CG gave up (internal error)");
   if (!S.h_mctl->all_done) throw Failure(HECMW33_ERR_TIMEOUT, "multi-RHS loop ended without a decision");
   if (S.h_mctl->fault) throw Failure(HECMW33_ERR_TIMEOUT, "multi-RHS SpMM: a bulk copy did not complete in time");
   for (int k = 0; k < nrhs; k++) {

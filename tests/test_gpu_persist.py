@@ -6,7 +6,7 @@ import pytest
 
 from frontistr_b200.matrix import HecMatrix
 from frontistr_b200.mesh import box_system
-from frontistr_b200.solver import GpuSolver
+from frontistr_b200.solver import GpuSolver, HecmwSolverError
 from oracle_ctypes import Oracle
 
 pytestmark = pytest.mark.gpu
@@ -216,3 +216,34 @@ def test_bicgstab_with_one_launch_applications(name):
     # BiCGSTAB carries rounding between its recurrences: the bounds of its own tests
     assert abs(rec["iter"] - ref["iter"]) <= max(3, ref["iter"] // 10)
     assert np.linalg.norm(m.X - ref["X"]) <= 1e-6 * np.linalg.norm(ref["X"])
+
+
+@pytest.mark.parametrize("call", ["cg16", "cg8", "cg4", "ilu", "multi", "bicgstab"])
+def test_barrier_that_gives_up_is_an_error(call, monkeypatch):
+    """A grid barrier whose polls run out (here after one) is reported whichever CTA gave up,
+    and the context stays usable."""
+    m = box_system(*{"cg8": (33, 31, 33), "cg4": (41, 39, 40), "ilu": (43, 40, 36)}.get(call, (14, 14, 20)))
+    m.set_iter(20)
+    if call == "ilu":
+        m.set_precond(10)
+    if call == "bicgstab":
+        m.set_method(2)
+
+    def solve(s):
+        if call != "multi":
+            m.X[:] = 0.0
+            return s.solve(m)
+        s.set_matrix(m)
+        X = np.zeros((3, 3 * m.N))
+        return s.solve_multi(np.tile(m.B, (3, 1)), X, m.Iarray, m.Rarray)
+
+    with GpuSolver() as s:
+        monkeypatch.setenv("HECMW33_BARRIER_POLLS", "1")
+        with pytest.raises(HecmwSolverError) as e:
+            solve(s)
+        assert e.value.code == 9103 and "gave up" in str(e.value)
+        monkeypatch.delenv("HECMW33_BARRIER_POLLS")
+        if call != "bicgstab":  # whose captured loop keeps its limit
+            assert solve(s)["error"] == 3001  # the iteration limit, as without the failure before it
+    with GpuSolver() as s:
+        assert solve(s)["error"] == 3001
