@@ -32,6 +32,7 @@ struct MrPersistArgs {
   const double *b;             // node order, 48 doubles per node
   double *x;                   // node order
   double *px, *r, *g, *p, *q, *h, *z, *u;  // position order
+  float *pl;                   // what p's rounding dropped, position order
   CgState *st;                 // kMaxRhs states out
   MultiCtl *ctl;
   const CgParams *prm;
@@ -167,31 +168,44 @@ __device__ __forceinline__ double mr_persist_sweep(const MrPersistArgs &a, MrSha
       x[2] = a8 * x[2];
       x[1] = a4 * (x[1] - a5 * x[2]);
       x[0] = a0 * (x[0] - a2 * x[2] - a1 * x[1]);
+      // the row's other vectors, their loads together (they took turns with the stores before:
+      // 16 cases on 118 thousand nodes 252 ms a solve, 226 so)
+      double f[3][5] = {};
+      float fl[3] = {};
+      if (MODE == 0 || (MODE == 1 && live)) {
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+          const size_t k = o + 16 * i;
+          f[i][0] = __ldcg((MODE == 0 ? a.r : a.g) + k);
+          if (MODE == 1) {
+            f[i][1] = __ldcg(a.z + k);
+            if (!first) {
+              f[i][2] = __ldcg(a.p + k);
+              f[i][3] = __ldcg(a.q + k);
+              f[i][4] = __ldcg(a.h + k);
+              fl[i] = __ldcg(a.pl + k);
+            }
+          }
+        }
+      }
 #pragma unroll
       for (int i = 0; i < 3; i++) {
         const size_t k = o + 16 * i;
+        a.u[k] = MODE == 0 ? lu_[i] : x[i];
         if (MODE == 0) {  // z = D^-1 (g - U z) and v = U z
           a.z[k] = x[i];
-          a.u[k] = lu_[i];
-          dot += __ldcg(a.r + k) * x[i];
+          dot += f[i][0] * x[i];
         } else if (MODE == 2) {
-          a.u[k] = x[i];
           if (again) a.g[k] = e[i];
-        } else {
-          a.u[k] = x[i];
-          if (live) {
-            const double gi = __ldcg(a.g + k);
-            double pn = __ldcg(a.z + k), qn = gi + lz[i], hn = gi - lu_[i];
-            if (!first) {
-              pn = pn + beta * __ldcg(a.p + k);
-              qn = qn + beta * __ldcg(a.q + k);
-              hn = hn + beta * __ldcg(a.h + k);
-            }
-            a.p[k] = pn;
-            a.q[k] = qn;
-            a.h[k] = hn;
-            dot += pn * qn;
-          }
+        } else if (live) {
+          float rest;  // first: BETA and the old vectors are zero
+          const double pn = next_direction(f[i][1], beta, f[i][2], fl[i], rest);
+          const double qn = f[i][0] + lz[i] + beta * f[i][3], hn = f[i][0] - lu_[i] + beta * f[i][4];
+          a.p[k] = pn;
+          a.pl[k] = rest;
+          a.q[k] = qn;
+          a.h[k] = hn;
+          dot += pn * qn;
         }
       }
       row += nhw;

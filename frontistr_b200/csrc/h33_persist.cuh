@@ -19,6 +19,15 @@
 // and tests on them); every true-residual refresh recomputes g from the new r by a plain
 // forward sweep.
 //
+// Rounding: hecmw_solve_CG's q is the product with the very p that goes into x.  Here q
+// follows z, so what p = z + BETA p loses to rounding would be missing from q for as long
+// as the direction lives, and the gap between r and b - A x grew to 1.6-1.9 times
+// hecmw_solve_CG's on slender boxes, 5 times on a chain with stiffness growing to 1e6 (64
+// bits, CPU, geometric means over loads).  p's lost part is therefore kept beside it, in
+// FP32 (pl: p to some 77 bits): 1.0-1.3 times, as wide as the scatter between loads.
+// Keeping q's part as well changed nothing more; q from a product at every refresh alone
+// left 1.5-1.8.
+//
 // What bounds it: the colours are a chain of 2 x NColor dependent steps.  As one launch
 // per colour a step cost 5 to 10 us whatever its size (launch, ramp, tail); here one CTA
 // per SM stays for the whole solve and a grid barrier (1.1 us bare, 1.6 us with the
@@ -64,6 +73,7 @@ struct SsorVecs {
   int n;
   double *r, *g, *p, *q, *h;
   double2 *zu;        // per position z and v (backward sweep) or u (forward): 3 double2
+  float *pl;          // what p's rounding dropped
 };
 
 struct PersistArgs {
@@ -214,6 +224,18 @@ struct GroupCursor {
   }
 };
 
+// p = z + BETA (p + pl): p rounded, the new pl in `rest`.  The product is split exactly, the
+// sum by the short form, which is exact for |BETA p| >= |z| and else misses a rounding of
+// z, as q misses one of A z.  None of it may be contracted.
+__device__ __forceinline__ double next_direction(double z, double beta, double p, float pl, float &rest) {
+  const double bp = __dmul_rn(beta, p), s = __dadd_rn(bp, z);
+  const double es = __dsub_rn(z, __dsub_rn(s, bp));
+  const double lo = __dadd_rn(es, fma(beta, double(pl), fma(beta, p, -bp)));
+  const double pn = __dadd_rn(s, lo);
+  rest = float(__dsub_rn(lo, __dsub_rn(pn, s)));
+  return pn;
+}
+
 // One sweep, MODE 0 backward, 1 forward on the direction, 2 forward from r (start and
 // refresh): the colours in turn, a barrier between them.  K lanes per row; lane c < 3 of
 // a row (MODE 1, K >= 8: of each half of its lanes) carries component c of its vectors.
@@ -245,6 +267,7 @@ __device__ __forceinline__ double ssor_sweep(const SsorVecs &a, const double *va
       const double a6 = __ldcs(lu + 6 * n), a7 = __ldcs(lu + 7 * n), a8 = __ldcs(lu + 8 * n);
       double o0, o1, o2;  // the row's own right-hand side: g, v or r
       double f0 = 0.0, f1 = 0.0, f2 = 0.0, f3 = 0.0, f4 = 0.0;
+      float fl = 0.0f;
       const double *own = reinterpret_cast<const double *>(a.zu + 3 * size_t(row));
       if (MODE == 1) {
         o0 = __ldcg(own + 3), o1 = __ldcg(own + 4), o2 = __ldcg(own + 5);
@@ -253,7 +276,10 @@ __device__ __forceinline__ double ssor_sweep(const SsorVecs &a, const double *va
           if (!first) f1 = __ldcg((up ? a.q : a.h) + i3 + c0);
           if (up) {
             f2 = __ldcg(own + c0);
-            if (!first) f3 = __ldcg(a.p + i3 + c0);
+            if (!first) {
+              f3 = __ldcg(a.p + i3 + c0);
+              fl = __ldcg(a.pl + i3 + c0);
+            }
           }
         } else {
           f2 = __ldcg(own + c0);
@@ -261,6 +287,7 @@ __device__ __forceinline__ double ssor_sweep(const SsorVecs &a, const double *va
             f1 = __ldcg(a.h + i3 + c0);
             f3 = __ldcg(a.p + i3 + c0);
             f4 = __ldcg(a.q + i3 + c0);
+            fl = __ldcg(a.pl + i3 + c0);
           }
         }
       } else {
@@ -311,6 +338,11 @@ __device__ __forceinline__ double ssor_sweep(const SsorVecs &a, const double *va
         for (int u = 0; u < U; u++)
           if (u < nx.y) col[u] = __ldg(cols + (nx.x + u) * 32 + lane);
       }
+      // the direction here, beside the lane sums: after them its chain would be the step's
+      // tail (first: BETA, p and pl are zero)
+      float rest = 0.0f;
+      double pn = 0.0;
+      if (MODE == 1) pn = next_direction(f2, beta, f3, fl, rest);
       if (HALVES) {
 #pragma unroll
         for (int j = 0; j < 3; j++) {
@@ -350,22 +382,22 @@ __device__ __forceinline__ double ssor_sweep(const SsorVecs &a, const double *va
           const double tn = first ? t : t + beta * f1;
           (up ? a.q : a.h)[i] = tn;
           if (up) {
-            const double pn = first ? f2 : f2 + beta * f3;
             a.p[i] = pn;
+            a.pl[i] = rest;
             dot += pn * tn;
           } else {
             *uo = xc;
           }
         } else {
           const double mc = cc == 0 ? m[0] : cc == 1 ? m[1] : m[2];
-          double pn = f2, qn = f0 + mc, hn = f0 - lc;
+          double qn = f0 + mc, hn = f0 - lc;
           if (!first) {
-            pn = pn + beta * f3;
             qn = qn + beta * f4;
             hn = hn + beta * f1;
           }
           *uo = xc;
           a.p[i] = pn;
+          a.pl[i] = rest;
           a.q[i] = qn;
           a.h[i] = hn;
           dot += pn * qn;

@@ -107,6 +107,7 @@ struct Batch {
   BatchArgs *h_args = nullptr;
   DevArray<double> b, x, r, z, p, q;
   DevArray<double> zu, g, h, px;  // position order (the fused iteration; zu also the unfused sweeps' intermediate)
+  DevArray<float> pl;             // the fused iteration's SsorVecs::pl
   DevArray<int> iperm;
   DevArray<int4> lo_desc, up_desc;
   // schedule and statistics
@@ -373,8 +374,10 @@ void batch_set_matrix(Batch &B, int nsys, const int *sys_ptr, int N, int NP, int
     const size_t n3 = size_t(3) * N;
     for (auto *v : {&B.b, &B.x, &B.r, &B.z, &B.p, &B.q}) v->alloc(n3);
     B.zu.alloc(2 * n3);
-    if (kind == 1)
+    if (kind == 1) {
       for (auto *v : {&B.g, &B.h, &B.px}) v->alloc(n3);
+      B.pl.alloc(n3);
+    }
     B.out.alloc(size_t(nsys));
     if (B.h_out) cudaFreeHost(B.h_out);
     B.h_out = nullptr;
@@ -571,7 +574,8 @@ float run_batch(Batch &B, const Schedule &sc, int iterpremax, double tol, int ma
   a.iperm = B.iperm.p;
   a.zpos = B.zu.p;
   a.px = B.px.p;
-  a.v = SsorVecs{B.alu.p, B.N, B.r.p, B.g.p, B.p.p, B.q.p, B.h.p, reinterpret_cast<double2 *>(B.zu.p)};
+  a.v = SsorVecs{B.alu.p, B.N, B.r.p, B.g.p, B.p.p, B.q.p, B.h.p, reinterpret_cast<double2 *>(B.zu.p),
+                 B.pl.p};
   a.out = B.out.p;
   a.tol = tol;
   a.maxit = maxit;

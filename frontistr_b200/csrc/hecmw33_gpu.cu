@@ -302,6 +302,7 @@ struct PersistPlan {
   DevArray<int4> lo_items, up_items;
   DevArray<int> iperm;
   DevArray<double> zu, parts;
+  DevArray<float> pl;
   DevArray<unsigned> bar;
 };
 
@@ -310,6 +311,7 @@ struct MrPersistPlan {
   int generation = -1;  // Precond::generation it was made for
   DevArray<int> rows, lo_gs, up_gs, iperm;
   DevArray<double> z, u, parts;
+  DevArray<float> pl;
   DevArray<unsigned> bar;
 };
 
@@ -1944,6 +1946,7 @@ void persist_plan(Solver &S) {
              L.iperm.p);
     H33_CUDA(cudaGetLastError());
     L.zu.alloc(6 * size_t(S.N));
+    L.pl.alloc(3 * size_t(S.N));
   }
   L.parts.alloc(3 * size_t(L.grid));
   L.bar.alloc(8);  // [0, 1] the CG's, [4, 6] the single application's
@@ -2009,7 +2012,8 @@ float run_cg_persist(Solver &S, double tol, int maxit, int *kernels) {
   } else {  // the solve's work vectors, here in position order
     a.px = S.w.p;
     a.pr = S.zp.p;
-    a.v = SsorVecs{P.alu_fwd.p, S.N, a.pr, S.z.p, a.pp, a.pq, S.zpos.p, reinterpret_cast<double2 *>(L.zu.p)};
+    a.v = SsorVecs{P.alu_fwd.p, S.N, a.pr, S.z.p, a.pp, a.pq, S.zpos.p, reinterpret_cast<double2 *>(L.zu.p),
+                   L.pl.p};
   }
   a.st = S.state.p;
   a.prm = S.params.p;
@@ -4248,6 +4252,7 @@ void run_mr_persist(Solver &S, int nrhs) {
     H33_CUDA(cudaGetLastError());
     L.z.alloc(n48);
     L.u.alloc(n48);
+    L.pl.alloc(n48);
     L.parts.alloc(3 * size_t(S.nsm) * kMaxRhs);
     L.bar.alloc(2);
     S.sync();
@@ -4273,6 +4278,7 @@ void run_mr_persist(Solver &S, int nrhs) {
   a.h = S.mzpos.p;
   a.z = L.z.p;
   a.u = L.u.p;
+  a.pl = L.pl.p;
   a.st = S.mst.p;
   a.ctl = S.mctl.p;
   a.prm = S.params.p;
