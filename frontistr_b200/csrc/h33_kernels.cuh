@@ -371,6 +371,28 @@ __global__ void pack_sell_kernel(T *__restrict__ val, const int *__restrict__ sr
   }
 }
 
+// The blocks of a sliced layout back in their raw places.
+static __global__ void unpack_sell_kernel(const double *__restrict__ val, const int *__restrict__ src, int nslots,
+                                          double *__restrict__ raw) {
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nslots * 32; t += gridDim.x * blockDim.x) {
+    const int b = src[t];
+    if (b < 0) continue;
+    const double *v = val + size_t(t >> 5) * 288 + (t & 31);
+#pragma unroll
+    for (int e = 0; e < 9; e++) raw[9 * size_t(b) + e] = v[e * 32];
+  }
+}
+
+// The diagonal LU of positions iperm_old[node] at those of perm_new.
+static __global__ void reorder_alu_kernel(const double *__restrict__ old, const int *__restrict__ iperm_old,
+                                          const int *__restrict__ perm_new, int n, double *__restrict__ alu) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const int o = iperm_old[perm_new[i]];
+#pragma unroll
+    for (int e = 0; e < 9; e++) alu[size_t(e) * n + i] = old[size_t(e) * n + o];
+  }
+}
+
 // ALU for position `pos` from the diagonal block of node perm[pos]: sigma-scaled
 // diagonal, in-place LU with reciprocal pivots (hecmw_precond_SSOR_33.F90:157-208).
 // With lu_done != 0 the raw blocks are already factorised (block ILU(0)).

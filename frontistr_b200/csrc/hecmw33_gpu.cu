@@ -172,11 +172,16 @@ int sweep_lanes() {
   return (k == 4 || k == 8 || k == 16) ? k : 4;
 }
 
-// The same for the SSOR of a CG solve, whose rows per colour (n / ncolor) decide: the more
+// The same for the preconditioner of a CG solve, whose rows per colour (n / ncolor) decide: the more
 // lanes a row has the shorter a step of cg_ssor_persist_kernel, until its slices are
 // about half as many as the grid's warps (12 a CTA).  Measured per iteration with
 // 4 / 8 / 16 lanes (us): 1,105 rows a colour 133 / 115 / 108, 3,135 rows 146 / 126 / 145,
-// 7,350 rows 171 / 182 / 235, 17 thousand 272 / 317.
+// 7,350 rows 171 / 182 / 235, 17 thousand 272 / 317.  The CG loops that keep a launch per
+// colour take the same lanes and are faster with them than with 4; us per iteration with
+// 4 / 8 / 16 at 22, 1,105, 2,657 and 7,350 rows a colour: SIGMA_DIAG 1.2 181 / 151 / 137,
+// 305 / 253 / 220, 346 / 274 / 230, 378 / 307 / 278 (with BF16 sweeps 169 / 142 / 131 to
+// 287 / 252 / 245); two passes 298 / 245 / 217 to 675 / 529 / 466; the FP32 inner CG of
+// precision mode 3 154 / 135 / 129 to 285 / 245 / 237.
 int ssor_lanes(int n, int ncolor, int nsm) {
   if (std::getenv("HECMW33_SWEEP_LANES")) return sweep_lanes();
   const int64_t rows = n / std::max(ncolor, 1);
@@ -190,6 +195,13 @@ int barrier_polls() {
   const char *e = std::getenv("HECMW33_BARRIER_POLLS");
   return e ? std::max(1, std::atoi(e)) : 1 << 23;
 }
+
+// Lanes per row of a layout with `groups` colours or levels, for CG (cg) or another method.
+// BiCGSTAB, GMRES and the others keep sweep_lanes(): their iterations depend on the
+// sweeps' rounding, and with launches per colour they lose more than they win (BiCGSTAB at
+// 1,105 / 2,657 / 7,350 rows a colour 356 / 377 / 455 us an iteration in one launch per
+// application with 4 lanes, 424 / 460 / 531 with 8, 357 / 378 / 470 with 16).
+int loop_lanes(int n, int groups, int nsm, bool cg) { return cg ? ssor_lanes(n, groups, nsm) : sweep_lanes(); }
 
 double wall() {
   return std::chrono::duration<double>(std::chrono::steady_clock::now().time_since_epoch()).count();
@@ -937,11 +949,104 @@ void diag_alu(Solver &S, DevArray<double> &alu, const double *blocks, const int 
   H33_CUDA(cudaGetLastError());
 }
 
+// The SSOR layouts of P with `lanes` lanes per row, from its ordering (P.perm, P.colorindex).
+void ssor_layout(Solver &S, Precond &P, int lanes) {
+  const Profile prof{S.N, S.indexL.data(), S.itemL.data(), S.indexU.data(), S.itemU.data()};
+  const std::vector<int> &perm = P.perm, &colorindex = P.colorindex;
+  std::vector<int> iperm(perm.size());
+  for (size_t i = 0; i < perm.size(); i++) iperm[size_t(perm[i])] = int(i);
+  if (host_layouts()) {
+    BlockRows lower_ref, upper_ref, lower, upper;
+    reordered_rows(prof, perm, iperm, lower_ref, upper_ref);
+    // the device sweeps gather from their colour-ordered intermediate: columns as
+    // positions (the same blocks in the same order; only the index names change)
+    for (auto *br : {&lower_ref, &upper_ref})
+      for (int &c : br->col) c = iperm[c];
+    // inside each colour the device places its rows by slot count (rows of one
+    // colour never read each other, so the sweep's arithmetic per row is unchanged):
+    // the slices of a colour then need few distinct slot counts and little padding
+    std::vector<int> order, iorder(size_t(S.N));
+    order_rows_by_length(lower_ref, upper_ref, colorindex, lanes, order);
+    for (int i = 0; i < S.N; i++) iorder[size_t(order[size_t(i)])] = i;
+    permute_rows(lower_ref, order, iorder, lower);
+    permute_rows(upper_ref, order, iorder, upper);
+    std::vector<int> perm_dev(size_t(S.N));
+    for (int i = 0; i < S.N; i++) perm_dev[size_t(i)] = perm[size_t(order[size_t(i)])];
+    SellLayout lo, up;
+    build_sell(lower, colorindex, lo, lanes, kMaxRuns);
+    build_sell(upper, colorindex, up, lanes, kMaxRuns);
+    P.lo.upload(lo, S.stream);
+    P.up.upload(up, S.stream);
+    P.perm_fwd.upload(perm_dev, S.stream);
+  } else {
+    // the same layouts with the O(blocks) work on the device: the rows' lower and
+    // upper block counts in the new order (count_parts_kernel), the row order inside
+    // each colour and the layouts' shape from those counts on the host, the blocks
+    // placed by fill_reordered_kernel
+    const int N = S.N;
+    const DevProfile dp = dev_profile(S);
+    DevArray<int> d_perm, d_iperm, d_nl, d_nu, d_order, d_iorder, d_row_slice;
+    d_perm.upload(perm, S.stream);
+    d_iperm.upload(iperm, S.stream);
+    d_nl.alloc(size_t(N));
+    d_nu.alloc(size_t(N));
+    const int grid = std::max(1, std::min((N + kThreads - 1) / kThreads, S.nsm * 8));
+    launch_k(S.stream, count_parts_kernel, grid, kThreads, dp, static_cast<const int *>(d_iperm.p), d_nl.p, d_nu.p);
+    H33_CUDA(cudaGetLastError());
+    std::vector<int> nl(static_cast<size_t>(N)), nu(static_cast<size_t>(N));
+    H33_CUDA(cudaMemcpyAsync(nl.data(), d_nl.p, sizeof(int) * size_t(N), cudaMemcpyDeviceToHost, S.stream));
+    H33_CUDA(cudaMemcpyAsync(nu.data(), d_nu.p, sizeof(int) * size_t(N), cudaMemcpyDeviceToHost, S.stream));
+    S.sync();
+    setup_mark("  ssor layouts: row counts (device)");
+    const size_t nn = static_cast<size_t>(N);
+    std::vector<int> order, iorder(nn), cl(nn), cu(nn), perm_dev(nn);
+    order_rows_by_counts(nl.data(), nu.data(), N, colorindex, lanes, order);
+    for (int q = 0; q < N; q++) {
+      const int i = order[size_t(q)];
+      iorder[size_t(i)] = q;
+      cl[size_t(q)] = nl[size_t(i)];
+      cu[size_t(q)] = nu[size_t(i)];
+      perm_dev[size_t(q)] = perm[size_t(i)];
+    }
+    SellLayout lo, up;
+    sell_shape(cl.data(), colorindex, lo, lanes, kMaxRuns);
+    sell_shape(cu.data(), colorindex, up, lanes, kMaxRuns);
+    // both parts cut the colours into the same slices (same groups, same rows per slice)
+    std::vector<int> row_slice(nn);
+    for (int sl = 0; sl < lo.nslices; sl++)
+      for (int r = 0; r < lo.nrows[size_t(sl)]; r++) row_slice[size_t(lo.row0[size_t(sl)] + r)] = sl;
+    setup_mark("  ssor layouts: row order, shape (host)");
+    P.lo.upload_shape(lo, S.stream);
+    P.up.upload_shape(up, S.stream);
+    setup_mark("  ssor layouts: shape up, arrays allocated");
+    d_order.upload(order, S.stream);
+    d_iorder.upload(iorder, S.stream);
+    d_row_slice.upload(row_slice, S.stream);
+    const int gw = std::max(1, std::min((N + kWarpsPerCta - 1) / kWarpsPerCta, S.nsm * 8));
+    launch_k(S.stream, fill_reordered_kernel<true>, gw, kThreads, dp, static_cast<const int *>(d_perm.p),
+             static_cast<const int *>(d_iperm.p), static_cast<const int *>(d_order.p),
+             static_cast<const int *>(d_iorder.p), static_cast<const int *>(d_row_slice.p),
+             static_cast<const int *>(P.lo.row0.p), static_cast<const int *>(P.lo.slot0.p), lanes, P.lo.col.p,
+             P.lo.src.p);
+    launch_k(S.stream, fill_reordered_kernel<false>, gw, kThreads, dp, static_cast<const int *>(d_perm.p),
+             static_cast<const int *>(d_iperm.p), static_cast<const int *>(d_order.p),
+             static_cast<const int *>(d_iorder.p), static_cast<const int *>(d_row_slice.p),
+             static_cast<const int *>(P.up.row0.p), static_cast<const int *>(P.up.slot0.p), lanes, P.up.col.p,
+             P.up.src.p);
+    H33_CUDA(cudaGetLastError());
+    P.perm_fwd.upload(perm_dev, S.stream);
+    S.sync();  // the fills read the temporaries above
+    setup_mark("  ssor layouts: blocks placed (device)");
+  }
+  P.lo.group_rows = colorindex;
+  P.up.group_rows = colorindex;
+  setup_mark("ssor: layouts");
+}
+
 // SSOR in P: the reference's RCM + multicolour ordering (greedy = false, the drop-in),
 // or first-fit colours in the input order (greedy = true: the learned preconditioner's
 // smoother, which is not bound to the reference's schedule).
-// cg: the lanes per row are the persistent CG's; the other methods and the smoother keep
-// sweep_lanes() for the launches per colour.
+// cg: the lanes per row are CG's (loop_lanes).
 void setup_ssor(Solver &S, Precond &P, int ncolor_in, double sigma, bool symbolic, bool greedy, bool cg) {
   P.sigma = sigma;
   if (symbolic) {
@@ -957,99 +1062,13 @@ void setup_ssor(Solver &S, Precond &P, int ncolor_in, double sigma, bool symboli
       P.ncolor = ordering_mc(prof, perm_rcm, ncolor_in, colorindex, perm, iperm);
       setup_mark("ssor: multicolouring");
     }
-    const int lanes = cg ? ssor_lanes(S.N, P.ncolor, S.nsm) : sweep_lanes();
-    if (host_layouts()) {
-      BlockRows lower_ref, upper_ref, lower, upper;
-      reordered_rows(prof, perm, iperm, lower_ref, upper_ref);
-      // the device sweeps gather from their colour-ordered intermediate: columns as
-      // positions (the same blocks in the same order; only the index names change)
-      for (auto *br : {&lower_ref, &upper_ref})
-        for (int &c : br->col) c = iperm[c];
-      // inside each colour the device places its rows by slot count (rows of one
-      // colour never read each other, so the sweep's arithmetic per row is unchanged):
-      // the slices of a colour then need few distinct slot counts and little padding
-      std::vector<int> order, iorder(size_t(S.N));
-      order_rows_by_length(lower_ref, upper_ref, colorindex, lanes, order);
-      for (int i = 0; i < S.N; i++) iorder[size_t(order[size_t(i)])] = i;
-      permute_rows(lower_ref, order, iorder, lower);
-      permute_rows(upper_ref, order, iorder, upper);
-      std::vector<int> perm_dev(size_t(S.N));
-      for (int i = 0; i < S.N; i++) perm_dev[size_t(i)] = perm[size_t(order[size_t(i)])];
-      SellLayout lo, up;
-      build_sell(lower, colorindex, lo, lanes, kMaxRuns);
-      build_sell(upper, colorindex, up, lanes, kMaxRuns);
-      P.lo.upload(lo, S.stream);
-      P.up.upload(up, S.stream);
-      P.perm_fwd.upload(perm_dev, S.stream);
-    } else {
-      // the same layouts with the O(blocks) work on the device: the rows' lower and
-      // upper block counts in the new order (count_parts_kernel), the row order inside
-      // each colour and the layouts' shape from those counts on the host, the blocks
-      // placed by fill_reordered_kernel
-      const int N = S.N;
-      const DevProfile dp = dev_profile(S);
-      DevArray<int> d_perm, d_iperm, d_nl, d_nu, d_order, d_iorder, d_row_slice;
-      d_perm.upload(perm, S.stream);
-      d_iperm.upload(iperm, S.stream);
-      d_nl.alloc(size_t(N));
-      d_nu.alloc(size_t(N));
-      const int grid = std::max(1, std::min((N + kThreads - 1) / kThreads, S.nsm * 8));
-      launch_k(S.stream, count_parts_kernel, grid, kThreads, dp, static_cast<const int *>(d_iperm.p), d_nl.p, d_nu.p);
-      H33_CUDA(cudaGetLastError());
-      std::vector<int> nl(static_cast<size_t>(N)), nu(static_cast<size_t>(N));
-      H33_CUDA(cudaMemcpyAsync(nl.data(), d_nl.p, sizeof(int) * size_t(N), cudaMemcpyDeviceToHost, S.stream));
-      H33_CUDA(cudaMemcpyAsync(nu.data(), d_nu.p, sizeof(int) * size_t(N), cudaMemcpyDeviceToHost, S.stream));
-      S.sync();
-      setup_mark("  ssor layouts: row counts (device)");
-      const size_t nn = static_cast<size_t>(N);
-      std::vector<int> order, iorder(nn), cl(nn), cu(nn), perm_dev(nn);
-      order_rows_by_counts(nl.data(), nu.data(), N, colorindex, lanes, order);
-      for (int q = 0; q < N; q++) {
-        const int i = order[size_t(q)];
-        iorder[size_t(i)] = q;
-        cl[size_t(q)] = nl[size_t(i)];
-        cu[size_t(q)] = nu[size_t(i)];
-        perm_dev[size_t(q)] = perm[size_t(i)];
-      }
-      SellLayout lo, up;
-      sell_shape(cl.data(), colorindex, lo, lanes, kMaxRuns);
-      sell_shape(cu.data(), colorindex, up, lanes, kMaxRuns);
-      // both parts cut the colours into the same slices (same groups, same rows per slice)
-      std::vector<int> row_slice(nn);
-      for (int sl = 0; sl < lo.nslices; sl++)
-        for (int r = 0; r < lo.nrows[size_t(sl)]; r++) row_slice[size_t(lo.row0[size_t(sl)] + r)] = sl;
-      setup_mark("  ssor layouts: row order, shape (host)");
-      P.lo.upload_shape(lo, S.stream);
-      P.up.upload_shape(up, S.stream);
-      setup_mark("  ssor layouts: shape up, arrays allocated");
-      d_order.upload(order, S.stream);
-      d_iorder.upload(iorder, S.stream);
-      d_row_slice.upload(row_slice, S.stream);
-      const int gw = std::max(1, std::min((N + kWarpsPerCta - 1) / kWarpsPerCta, S.nsm * 8));
-      launch_k(S.stream, fill_reordered_kernel<true>, gw, kThreads, dp, static_cast<const int *>(d_perm.p),
-               static_cast<const int *>(d_iperm.p), static_cast<const int *>(d_order.p),
-               static_cast<const int *>(d_iorder.p), static_cast<const int *>(d_row_slice.p),
-               static_cast<const int *>(P.lo.row0.p), static_cast<const int *>(P.lo.slot0.p), lanes, P.lo.col.p,
-               P.lo.src.p);
-      launch_k(S.stream, fill_reordered_kernel<false>, gw, kThreads, dp, static_cast<const int *>(d_perm.p),
-               static_cast<const int *>(d_iperm.p), static_cast<const int *>(d_order.p),
-               static_cast<const int *>(d_iorder.p), static_cast<const int *>(d_row_slice.p),
-               static_cast<const int *>(P.up.row0.p), static_cast<const int *>(P.up.slot0.p), lanes, P.up.col.p,
-               P.up.src.p);
-      H33_CUDA(cudaGetLastError());
-      P.perm_fwd.upload(perm_dev, S.stream);
-      S.sync();  // the fills read the temporaries above
-      setup_mark("  ssor layouts: blocks placed (device)");
-    }
-    setup_mark("ssor: layouts");
+    P.colorindex = colorindex;
+    P.perm = perm;  // the reference's ordering (reported); the device uses perm_dev
+    ssor_layout(S, P, loop_lanes(S.N, P.ncolor, S.nsm, cg));
     P.pos_cols = true;
     // padding blocks gather zpos[0]: it must hold finite values from the start
     S.zpos.alloc(size_t(3) * S.N);
     S.zpos.zero(S.stream);
-    P.lo.group_rows = colorindex;
-    P.up.group_rows = colorindex;
-    P.colorindex = colorindex;
-    P.perm = perm;  // the reference's ordering (reported); the device uses perm_dev
     P.alu_shared = true;
   }
   P.lo.pack(S.raw.p, S.stream, S.nsm);
@@ -1057,6 +1076,89 @@ void setup_ssor(Solver &S, Precond &P, int ncolor_in, double sigma, bool symboli
   diag_alu(S, P.alu_fwd, S.raw.p, P.perm_fwd.p, sigma, 0);
   P.values_version = S.values_version;
   setup_mark("ssor: value packing + diagonal LU");
+}
+
+// The block ILU's layouts in the level schedules of its factor pattern.
+void bilu_layout(Solver &S, Precond &P, bool cg) {
+  const Profile prof = P.ilu_level > 0
+                           ? P.fill.view()
+                           : Profile{S.N, S.indexL.data(), S.itemL.data(), S.indexU.data(), S.itemU.data()};
+  std::vector<int> ord_f, lev_f, ord_b, lev_b;
+  level_schedule(prof, true, ord_f, lev_f);
+  level_schedule(prof, false, ord_b, lev_b);
+  const int lanes = loop_lanes(S.N, int(lev_f.size()) - 1, S.nsm, cg);
+  if (P.ilu_level == 0 && !host_layouts()) {
+    // the matrix's own pattern: the shapes from the rows' counts, the blocks placed
+    // on the device from the resident profile (fill_ordered_kernel)
+    const int N = S.N;
+    const size_t nn = static_cast<size_t>(N);
+    std::vector<int> cl(nn), cu(nn);
+    for (int q = 0; q < N; q++) {
+      cl[size_t(q)] = S.indexL[size_t(ord_f[size_t(q)]) + 1] - S.indexL[size_t(ord_f[size_t(q)])];
+      cu[size_t(q)] = S.indexU[size_t(ord_b[size_t(q)]) + 1] - S.indexU[size_t(ord_b[size_t(q)])];
+    }
+    SellLayout lo, up;
+    sell_shape(cl.data(), lev_f, lo, lanes);
+    sell_shape(cu.data(), lev_b, up, lanes);
+    std::vector<int> rs_f(nn), rs_b(nn);
+    for (int sl = 0; sl < lo.nslices; sl++)
+      for (int r = 0; r < lo.nrows[size_t(sl)]; r++) rs_f[size_t(lo.row0[size_t(sl)] + r)] = sl;
+    for (int sl = 0; sl < up.nslices; sl++)
+      for (int r = 0; r < up.nrows[size_t(sl)]; r++) rs_b[size_t(up.row0[size_t(sl)] + r)] = sl;
+    P.lo.upload_shape(lo, S.stream);
+    P.up.upload_shape(up, S.stream);
+    P.perm_fwd.upload(ord_f, S.stream);
+    P.perm_bwd.upload(ord_b, S.stream);
+    DevArray<int> d_rsf, d_rsb;
+    d_rsf.upload(rs_f, S.stream);
+    d_rsb.upload(rs_b, S.stream);
+    const DevProfile dp = dev_profile(S);
+    const int grid = std::max(1, std::min((N + kThreads - 1) / kThreads, S.nsm * 8));
+    launch_k(S.stream, fill_ordered_kernel<false>, grid, kThreads, dp, static_cast<const int *>(P.perm_fwd.p),
+             static_cast<const int *>(d_rsf.p), static_cast<const int *>(P.lo.row0.p),
+             static_cast<const int *>(P.lo.slot0.p), lanes, P.lo.col.p, P.lo.src.p);
+    launch_k(S.stream, fill_ordered_kernel<true>, grid, kThreads, dp, static_cast<const int *>(P.perm_bwd.p),
+             static_cast<const int *>(d_rsb.p), static_cast<const int *>(P.up.row0.p),
+             static_cast<const int *>(P.up.slot0.p), lanes, P.up.col.p, P.up.src.p);
+    H33_CUDA(cudaGetLastError());
+    S.sync();  // the fills read the row-slice tables above
+  } else {  // the filled pattern of ILU(1)/(2), or HECMW33_HOST_LAYOUT=1: on the host
+    BlockRows lower, upper;
+    const int N = S.N, NPL = prof.NPL();
+    lower.ptr.assign(size_t(N) + 1, 0);
+    upper.ptr.assign(size_t(N) + 1, 0);
+    for (int pos = 0; pos < N; pos++) {
+      const int i = ord_f[pos];
+      lower.ptr[pos + 1] = lower.ptr[pos] + (prof.indexL[i + 1] - prof.indexL[i]);
+      const int k = ord_b[pos];
+      upper.ptr[pos + 1] = upper.ptr[pos] + (prof.indexU[k + 1] - prof.indexU[k]);
+    }
+    lower.col.resize(size_t(lower.ptr[N]));
+    lower.src.resize(size_t(lower.ptr[N]));
+    upper.col.resize(size_t(upper.ptr[N]));
+    upper.src.resize(size_t(upper.ptr[N]));
+    for (int pos = 0; pos < N; pos++) {
+      const int i = ord_f[pos];
+      int64_t w = lower.ptr[pos];
+      for (int j = prof.indexL[i]; j < prof.indexL[i + 1]; j++) {
+        lower.col[w] = prof.itemL[j] - 1;
+        lower.src[w++] = N + j;
+      }
+      const int k = ord_b[pos];
+      w = upper.ptr[pos];
+      for (int j = prof.indexU[k]; j < prof.indexU[k + 1]; j++) {
+        upper.col[w] = prof.itemU[j] - 1;
+        upper.src[w++] = N + NPL + j;
+      }
+    }
+    SellLayout lo, up;
+    build_sell(lower, lev_f, lo, lanes);
+    build_sell(upper, lev_b, up, lanes);
+    P.lo.upload(lo, S.stream);
+    P.up.upload(up, S.stream);
+    P.perm_fwd.upload(ord_f, S.stream);
+    P.perm_bwd.upload(ord_b, S.stream);
+  }
 }
 
 // Block ILU(p) (hecmw_precond_BILU_33.f90): p = 0 on the matrix's own pattern
@@ -1068,86 +1170,10 @@ void setup_bilu(Solver &S, int level, double sigma, bool symbolic, bool cg) {
   const Profile prof0{S.N, S.indexL.data(), S.itemL.data(), S.indexU.data(), S.itemU.data()};
   if (symbolic) {
     if (level > 0) bilu_fill(prof0, level, P.fill);
-    const Profile prof = level > 0 ? P.fill.view() : prof0;
-    std::vector<int> ord_f, lev_f, ord_b, lev_b;
-    level_schedule(prof, true, ord_f, lev_f);
-    level_schedule(prof, false, ord_b, lev_b);
-    const int lanes = cg ? ssor_lanes(S.N, int(lev_f.size()) - 1, S.nsm) : sweep_lanes();
-    if (level == 0 && !host_layouts()) {
-      // the matrix's own pattern: the shapes from the rows' counts, the blocks placed
-      // on the device from the resident profile (fill_ordered_kernel)
-      const int N = S.N;
-      const size_t nn = static_cast<size_t>(N);
-      std::vector<int> cl(nn), cu(nn);
-      for (int q = 0; q < N; q++) {
-        cl[size_t(q)] = S.indexL[size_t(ord_f[size_t(q)]) + 1] - S.indexL[size_t(ord_f[size_t(q)])];
-        cu[size_t(q)] = S.indexU[size_t(ord_b[size_t(q)]) + 1] - S.indexU[size_t(ord_b[size_t(q)])];
-      }
-      SellLayout lo, up;
-      sell_shape(cl.data(), lev_f, lo, lanes);
-      sell_shape(cu.data(), lev_b, up, lanes);
-      std::vector<int> rs_f(nn), rs_b(nn);
-      for (int sl = 0; sl < lo.nslices; sl++)
-        for (int r = 0; r < lo.nrows[size_t(sl)]; r++) rs_f[size_t(lo.row0[size_t(sl)] + r)] = sl;
-      for (int sl = 0; sl < up.nslices; sl++)
-        for (int r = 0; r < up.nrows[size_t(sl)]; r++) rs_b[size_t(up.row0[size_t(sl)] + r)] = sl;
-      P.lo.upload_shape(lo, S.stream);
-      P.up.upload_shape(up, S.stream);
-      P.perm_fwd.upload(ord_f, S.stream);
-      P.perm_bwd.upload(ord_b, S.stream);
-      DevArray<int> d_rsf, d_rsb;
-      d_rsf.upload(rs_f, S.stream);
-      d_rsb.upload(rs_b, S.stream);
-      const DevProfile dp = dev_profile(S);
-      const int grid = std::max(1, std::min((N + kThreads - 1) / kThreads, S.nsm * 8));
-      launch_k(S.stream, fill_ordered_kernel<false>, grid, kThreads, dp, static_cast<const int *>(P.perm_fwd.p),
-               static_cast<const int *>(d_rsf.p), static_cast<const int *>(P.lo.row0.p),
-               static_cast<const int *>(P.lo.slot0.p), lanes, P.lo.col.p, P.lo.src.p);
-      launch_k(S.stream, fill_ordered_kernel<true>, grid, kThreads, dp, static_cast<const int *>(P.perm_bwd.p),
-               static_cast<const int *>(d_rsb.p), static_cast<const int *>(P.up.row0.p),
-               static_cast<const int *>(P.up.slot0.p), lanes, P.up.col.p, P.up.src.p);
-      H33_CUDA(cudaGetLastError());
-      S.sync();  // the fills read the row-slice tables above
-    } else {  // the filled pattern of ILU(1)/(2), or HECMW33_HOST_LAYOUT=1: on the host
-      BlockRows lower, upper;
-      const int N = S.N, NPL = prof.NPL();
-      lower.ptr.assign(size_t(N) + 1, 0);
-      upper.ptr.assign(size_t(N) + 1, 0);
-      for (int pos = 0; pos < N; pos++) {
-        const int i = ord_f[pos];
-        lower.ptr[pos + 1] = lower.ptr[pos] + (prof.indexL[i + 1] - prof.indexL[i]);
-        const int k = ord_b[pos];
-        upper.ptr[pos + 1] = upper.ptr[pos] + (prof.indexU[k + 1] - prof.indexU[k]);
-      }
-      lower.col.resize(size_t(lower.ptr[N]));
-      lower.src.resize(size_t(lower.ptr[N]));
-      upper.col.resize(size_t(upper.ptr[N]));
-      upper.src.resize(size_t(upper.ptr[N]));
-      for (int pos = 0; pos < N; pos++) {
-        const int i = ord_f[pos];
-        int64_t w = lower.ptr[pos];
-        for (int j = prof.indexL[i]; j < prof.indexL[i + 1]; j++) {
-          lower.col[w] = prof.itemL[j] - 1;
-          lower.src[w++] = N + j;
-        }
-        const int k = ord_b[pos];
-        w = upper.ptr[pos];
-        for (int j = prof.indexU[k]; j < prof.indexU[k + 1]; j++) {
-          upper.col[w] = prof.itemU[j] - 1;
-          upper.src[w++] = N + NPL + j;
-        }
-      }
-      SellLayout lo, up;
-      build_sell(lower, lev_f, lo, lanes);
-      build_sell(upper, lev_b, up, lanes);
-      P.lo.upload(lo, S.stream);
-      P.up.upload(up, S.stream);
-      P.perm_fwd.upload(ord_f, S.stream);
-      P.perm_bwd.upload(ord_b, S.stream);
-    }
+    P.ilu_level = level;
+    bilu_layout(S, P, cg);
     P.alu_shared = false;
     P.ncolor = 0;
-    P.ilu_level = level;
   }
   // numeric factorisation on the host, from the resident values
   const size_t nb = size_t(S.N) + S.NPL + S.NPU;
@@ -1175,6 +1201,47 @@ void setup_bilu(Solver &S, int level, double sigma, bool symbolic, bool cg) {
   diag_alu(S, P.alu_fwd, P.ilu_raw.p, P.perm_fwd.p, 1.0, 1);
   diag_alu(S, P.alu_bwd, P.ilu_raw.p, P.perm_bwd.p, 1.0, 1);
   S.sync();
+}
+
+// Brings the layouts of the solve's preconditioner to the lanes per row of the loop that
+// is about to use it (CG's or another method's), so that a solve's speed and rounding do
+// not depend on what the handle solved before.  The values move as they are: a recycled
+// preconditioner is older than the matrix.
+void relane(Solver &S, bool cg) {
+  Precond &P = S.pc;
+  if (!P.valid || P.kind == 3) return;
+  const int lanes = loop_lanes(S.N, int(P.lo.group_slice.size()) - 1, S.nsm, cg);
+  if (P.lo.lanes == lanes) return;
+  const int grid = std::max(1, std::min((S.N + kThreads - 1) / kThreads, S.nsm * 8));
+  if (P.kind == 1) {
+    DevArray<double> raw;
+    raw.alloc(9 * (size_t(S.N) + S.NPL + S.NPU));
+    for (auto *d : {&P.lo, &P.up})
+      if (d->nslots) launch_k(S.stream, unpack_sell_kernel, grid, kThreads, static_cast<const double *>(d->val.p),
+                              static_cast<const int *>(d->src.p), d->nslots, raw.p);
+    DevArray<double> alu = std::move(P.alu_fwd);
+    DevArray<int> iperm;
+    iperm.alloc(size_t(S.N));
+    launch_k(S.stream, invert_perm_kernel, grid, kThreads, static_cast<const int *>(P.perm_fwd.p), S.N, iperm.p);
+    H33_CUDA(cudaGetLastError());
+    S.sync();  // the layout's arrays are made anew
+    ssor_layout(S, P, lanes);
+    P.lo.pack(raw.p, S.stream, S.nsm);
+    P.up.pack(raw.p, S.stream, S.nsm);
+    P.alu_fwd.alloc(alu.n);
+    launch_k(S.stream, reorder_alu_kernel, grid, kThreads, static_cast<const double *>(alu.p),
+             static_cast<const int *>(iperm.p), static_cast<const int *>(P.perm_fwd.p), S.N, P.alu_fwd.p);
+    H33_CUDA(cudaGetLastError());
+    S.sync();
+  } else {
+    bilu_layout(S, P, cg);
+    P.lo.pack(P.ilu_raw.p, S.stream, S.nsm);
+    P.up.pack(P.ilu_raw.p, S.stream, S.nsm);
+    S.sync();
+  }
+  P.fp32_version = P.lowp_version = -1;  // their copies were of the old layouts
+  P.generation = ++S.build_counter;
+  S.drop_graph();
 }
 
 // hecmw_mat_recycle_precond_setting (hecmw_matrix_misc.F90:858-877)
@@ -1209,8 +1276,9 @@ void precond_setup(Solver &S, int precond, int ncolor_in, double sigma, int *Iar
   const bool same = P.valid && P.kind == kind && (kind != 1 || P.ncolor_in == ncolor_in) &&
                     (kind != 10 || P.ilu_level == level);
   const bool reuse = same && Iarray[97] == 0 && Iarray[96] == 0;
-  if (reuse) return;
   const bool symbolic = !same;
+  if (!symbolic) relane(S, Iarray[1] == 1);
+  if (reuse) return;
   if (symbolic) {
     P = Precond();
   }
@@ -3665,8 +3733,11 @@ int solve_fp64(Solver &S, int *Iarray, double *Rarray, int *iter, double *resid,
     if (learned) ensure_lowp(S, S.L.sm);
     else ensure_lowp(S);
   }
-  S.apply_one = !persist() && !learned && !record && method != 1 && !lowp && iterPREmax > 0 && apply_rule(S);
-  if (S.apply_one) persist_plan<4>(S);
+  const auto choose_apply = [&] {
+    S.apply_one = !persist() && !learned && !record && method != 1 && !lowp && iterPREmax > 0 && apply_rule(S);
+    if (S.apply_one) persist_plan<4>(S);
+  };
+  choose_apply();
   struct ApplyScope {
     Solver &S;
     ~ApplyScope() { S.apply_one = false; }
@@ -3730,7 +3801,9 @@ int solve_fp64(Solver &S, int *Iarray, double *Rarray, int *iter, double *resid,
         if (auto_sigma) sigma = 1.0;
         method = METHOD2;
         learned = 0;
+        relane(S, false);
         if (lowp) ensure_lowp(S);
+        choose_apply();
         continue;
       }
     }

@@ -311,3 +311,40 @@ def test_attainable_accuracy_is_the_oracles(call, monkeypatch):
                     s.solve_resident(b, x, m.Iarray, m.Rarray)
     got = [true_resid(x, b) for x, b in zip(X, loads)]
     assert np.exp(np.mean(np.log(np.array(got) / np.array(ref)))) < 1.35
+
+
+@pytest.mark.parametrize("precond", [1, 10])
+@pytest.mark.parametrize("box", [(6, 5, 8), (14, 14, 20), (33, 31, 33)])
+def test_a_solve_does_not_depend_on_what_the_handle_solved_before(box, precond):
+    """CG and BiCGSTAB want different lanes per row: a handle that changes its method gives
+    the bits and the launches of a fresh one, and so does a recycled preconditioner, whose
+    values are older than the matrix."""
+    base = box_system(*box, jitter=0.2, sigma_E=1.0, nu_range=(0.25, 0.40), seed=5)
+    base.set_iter(60)  # a limit: what matters is the same arithmetic
+    base.set_precond(precond)
+
+    def run(methods):
+        m = base.copy()
+        out = []
+        with GpuSolver() as s:
+            for k, method in enumerate(methods):
+                m.set_method(method)
+                m.X[:] = 0.0
+                m.Iarray[96] = 2  # rebuilt
+                if k == len(methods) - 1:
+                    for a in (m.D, m.AL, m.AU):
+                        a *= 1.25
+                    m.Iarray[96] = 1  # new values, recycled preconditioner
+                rec = s.solve(m)
+                out.append((rec["iter"], s.last_solve_info()["kernels"], m.X.copy()))
+        return out
+
+    cg, bicg = run([1, 1]), run([2, 2])
+    mixed, back = run([1, 2, 1, 2]), run([2, 1])
+
+    def same(a, b):
+        return a[0] == b[0] and a[1] == b[1] and np.array_equal(a[2], b[2])
+
+    assert same(mixed[0], cg[0]) and same(mixed[1], bicg[0]) and same(mixed[2], cg[0])
+    assert same(mixed[3], bicg[1])
+    assert same(back[0], bicg[0]) and same(back[1], cg[1])
