@@ -20,7 +20,7 @@
 
 namespace h33 {
 
-constexpr int kMrWarps = 16;
+constexpr int kMrWarps = 16;  // most warps of a CTA
 constexpr int kMrThreads = 32 * kMrWarps;
 constexpr int kMrBlock = 5;  // double2 per staged block: nine entries and the column
 
@@ -48,7 +48,7 @@ struct MrShared {
   double res[kMaxRhs];
   int again[kMaxRhs];  // load cases whose g has to be made from r
   int any, dead;
-  double2 blk[2 * kMrWarps][16 * kMrBlock];
+  double2 blk[2 * kMrWarps][16 * kMrBlock];  // last: as many as the CTA has half-warps
 };
 
 __device__ __forceinline__ void mr_persist_barrier(const MrPersistArgs &a, MrShared &sh, unsigned &target) {
@@ -61,23 +61,23 @@ __device__ __forceinline__ void mr_persist_barrier(const MrPersistArgs &a, MrSha
 // Sum over the grid for every load case, in sh.res; includes a barrier.
 __device__ __forceinline__ void mr_persist_sum(const MrPersistArgs &a, MrShared &sh, unsigned &target, double v,
                                                int slot) {
-  const int l = threadIdx.x & 15, hw = threadIdx.x >> 4;
+  const int l = threadIdx.x & 15, hw = threadIdx.x >> 4, nh = blockDim.x >> 4;
   double *parts = a.parts + size_t(slot) * gridDim.x * kMaxRhs;
   sh.red[hw][l] = v;
   __syncthreads();
   if (threadIdx.x < kMaxRhs) {
     double s = 0.0;
-    for (int k = 0; k < 2 * kMrWarps; k++) s += sh.red[k][threadIdx.x];
+    for (int k = 0; k < nh; k++) s += sh.red[k][threadIdx.x];
     parts[size_t(blockIdx.x) * kMaxRhs + threadIdx.x] = s;
   }
   mr_persist_barrier(a, sh, target);
   double s = 0.0;
-  for (int i = hw; i < int(gridDim.x); i += 2 * kMrWarps) s += __ldcg(parts + size_t(i) * kMaxRhs + l);
+  for (int i = hw; i < int(gridDim.x); i += nh) s += __ldcg(parts + size_t(i) * kMaxRhs + l);
   sh.red[hw][l] = s;
   __syncthreads();
   if (threadIdx.x < kMaxRhs) {
     double t = 0.0;
-    for (int k = 0; k < 2 * kMrWarps; k++) t += sh.red[k][threadIdx.x];
+    for (int k = 0; k < nh; k++) t += sh.red[k][threadIdx.x];
     sh.res[threadIdx.x] = t;
   }
   __syncthreads();
@@ -137,7 +137,7 @@ template <int K, int MODE>
 __device__ __forceinline__ double mr_persist_sweep(const MrPersistArgs &a, MrShared &sh, unsigned &target) {
   constexpr int RPS = 32 / K;
   const int lane = threadIdx.x & 15, hwl = threadIdx.x >> 4;
-  const int hw = hwl * gridDim.x + blockIdx.x, nhw = 2 * kMrWarps * gridDim.x;
+  const int hw = hwl * gridDim.x + blockIdx.x, nhw = (blockDim.x >> 4) * gridDim.x;
   const unsigned hmask = (threadIdx.x & 16) ? 0xffff0000u : 0x0000ffffu;
   const SellView<double> &L = MODE == 0 ? a.up : a.lo;
   const int *gs = MODE == 0 ? a.up_gs : a.lo_gs;
@@ -222,7 +222,7 @@ __device__ __forceinline__ double mr_persist_sweep(const MrPersistArgs &a, MrSha
 template <bool BB>
 __device__ __forceinline__ double mr_persist_resid(const MrPersistArgs &a, MrShared &sh, bool mine) {
   const int lane = threadIdx.x & 15, hwl = threadIdx.x >> 4;
-  const int hw = hwl * gridDim.x + blockIdx.x, nhw = 2 * kMrWarps * gridDim.x;
+  const int hw = hwl * gridDim.x + blockIdx.x, nhw = (blockDim.x >> 4) * gridDim.x;
   const unsigned hmask = (threadIdx.x & 16) ? 0xffff0000u : 0x0000ffffu;
   double acc = 0.0;
   for (int row = hw; row < a.n; row += nhw) {
@@ -246,7 +246,7 @@ __global__ void __launch_bounds__(kMrThreads, 1) mr_cg_persist_kernel(const MrPe
   extern __shared__ __align__(16) unsigned char mr_smem[];
   MrShared &sh = *reinterpret_cast<MrShared *>(mr_smem);
   const int tid = threadIdx.x, lane = tid & 15;
-  const int hw = (tid >> 4) * gridDim.x + blockIdx.x, nhw = 2 * kMrWarps * gridDim.x;
+  const int hw = (tid >> 4) * gridDim.x + blockIdx.x, nhw = (blockDim.x >> 4) * gridDim.x;
   unsigned target = 0;
   if (tid < kMaxRhs) {
     CgState s = {};

@@ -306,10 +306,11 @@ struct Precond {
   int values_version = -1;  // matrix values (Solver::values_version) of the last numeric setup
 };
 
-// The persistent CG's per-warp slice lists and workspace for one SSOR layout.
+// The per-warp slice lists of one layout for the persistent CG, or for the single SSOR
+// application, and the CG's workspace.
 struct PersistPlan {
   int generation = -1;   // Precond::generation it was made for
-  int grid = 0, lo_stride = 0, up_stride = 0;
+  int grid = 0, warps = 0, lo_stride = 0, up_stride = 0;  // CTAs, warps of each
   bool cluster = false;
   DevArray<int4> lo_items, up_items;
   DevArray<int> iperm;
@@ -321,6 +322,7 @@ struct PersistPlan {
 // The same for several load cases.
 struct MrPersistPlan {
   int generation = -1;  // Precond::generation it was made for
+  int warps = 0;        // of a CTA
   DevArray<int> rows, lo_gs, up_gs, iperm;
   DevArray<double> z, u, parts;
   DevArray<float> pl;
@@ -471,7 +473,7 @@ struct Solver {
   unsigned *h_gave_up = nullptr;  // a one-launch solve's mark that a barrier gave up
   DevArray<int> d_err;
   Precond pc;
-  PersistPlan pp;
+  PersistPlan pp, ap;  // the one-launch CG's, the one-launch application's
   MrPersistPlan mpp;
   bool apply_one = false;  // this solve applies its SSOR in one launch (apply_rule)
   // FP32 copies for the mixed-precision refinement
@@ -1484,7 +1486,7 @@ void launch_sweep_t(Solver &S, const Precond &P, const SellView<TV> &lo, const S
 // colour launches / in one launch per application: 0.7 thousand nodes 299 / 238, 20
 // thousand 561 / 371, 36 thousand 612 / 382, 118 thousand (7,350 rows a colour) 675 / 456,
 // 275 thousand (17 thousand rows) 863 / 822; GMRES(30) on 20 thousand 494 / 371.
-// persist_plan<4> has to have run.
+// Its plan (S.ap) has to be there.
 bool apply_rule(const Solver &S) {
   const Precond &P = S.pc;
   return P.valid && P.kind == 1 && P.pos_cols && P.lo.lanes == 4 && S.N / std::max(P.ncolor, 1) <= 120 * S.nsm;
@@ -1492,12 +1494,12 @@ bool apply_rule(const Solver &S) {
 
 void launch_apply_persist(Solver &S, const double *rin, double *zout, double *zpos, const CgState *st) {
   const Precond &P = S.pc;
-  const PersistPlan &L = S.pp;
+  const PersistPlan &L = S.ap;
   ApplyArgs a{P.lo.view(), P.up.view(), L.lo_items.p, L.up_items.p, L.lo_stride, L.up_stride, P.perm_fwd.p,
-              P.alu_fwd.p, S.N, int(P.lo.group_slice.size()) - 1, rin, zout, zpos, st, L.bar.p + 4, barrier_polls()};
+              P.alu_fwd.p, S.N, int(P.lo.group_slice.size()) - 1, rin, zout, zpos, st, L.bar.p, barrier_polls()};
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(unsigned(L.grid), 1, 1);
-  cfg.blockDim = dim3(32 * persist_warps<4>(), 1, 1);
+  cfg.blockDim = dim3(unsigned(32 * L.warps), 1, 1);
   cfg.stream = S.stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeCooperative;
@@ -1984,15 +1986,29 @@ int persist_grid(Solver &S, bool ilu, int rows) {
   return S.nsm;
 }
 
+// Warps of a CTA of the single application: 4 while these have a slice each in the largest
+// colour, else all 16.  Alone it makes no difference, but four of 4 warps leave room beside
+// them for the launches of other handles; ms for one solve / for four handles at once, with
+// 16 warps and with 4: BiCGSTAB on 378 nodes 9.1 / 31 and 9.2 / 10.7, 19 thousand 106 / 409
+// and 107 / 129, 45 thousand 77 / 318 and 77 / 114 (as colour launches 11.3 / 12.5, 161 /
+// 216, 122 / 182); 118 thousand nodes need 7: 118 / 504 with 16, 119 / 657 with 7.
+int apply_warps(const Solver &S) {
+  const std::vector<int> &gs = S.pc.lo.group_slice;
+  int most = 0;
+  for (size_t g = 0; g + 1 < gs.size(); g++) most = std::max(most, gs[g + 1] - gs[g]);
+  return most <= 4 * S.nsm ? 4 : persist_warps<4>();
+}
+
+// apply: the plan of the single application.
 template <int K>
-void persist_plan(Solver &S) {
-  PersistPlan &L = S.pp;
+void persist_plan(Solver &S, PersistPlan &L, bool apply = false) {
   const Precond &P = S.pc;
   if (L.generation == P.generation) return;
-  const int grid = persist_grid<K>(S, P.kind == 10, S.N / std::max(int(P.lo.group_slice.size()) - 1, 1));
+  const int grid = apply ? S.nsm : persist_grid<K>(S, P.kind == 10, S.N / std::max(int(P.lo.group_slice.size()) - 1, 1));
   L.cluster = grid < 0;
   L.grid = std::abs(grid);
-  const int nw = L.grid * persist_warps<K>();
+  L.warps = apply ? apply_warps(S) : persist_warps<K>();
+  const int nw = L.grid * L.warps;
   auto lists = [&](const DevSell<double> &D, bool reverse, DevArray<int4> &items, int &stride) {
     const int ng = int(D.group_slice.size()) - 1;
     stride = 2;
@@ -2008,7 +2024,7 @@ void persist_plan(Solver &S) {
   };
   lists(P.lo, false, L.lo_items, L.lo_stride);
   lists(P.up, true, L.up_items, L.up_stride);
-  if (P.kind == 1) {
+  if (P.kind == 1 && !apply) {
     L.iperm.alloc(size_t(S.N));
     launch_k(S.stream, invert_perm_kernel, S.grid_vec(), kThreads, static_cast<const int *>(P.perm_fwd.p), S.N,
              L.iperm.p);
@@ -2017,7 +2033,7 @@ void persist_plan(Solver &S) {
     L.pl.alloc(3 * size_t(S.N));
   }
   L.parts.alloc(3 * size_t(L.grid));
-  L.bar.alloc(8);  // [0, 1] the CG's, [4, 6] the single application's
+  L.bar.alloc(4);
   L.bar.zero(S.stream);
   L.generation = P.generation;
 }
@@ -2042,9 +2058,9 @@ void launch_persist(Solver &S, const PersistArgs &a) {
 float run_cg_persist(Solver &S, double tol, int maxit, int *kernels) {
   const Precond &P = S.pc;
   switch (P.lo.lanes) {
-    case 8: persist_plan<8>(S); break;
-    case 16: persist_plan<16>(S); break;
-    default: persist_plan<4>(S); break;
+    case 8: persist_plan<8>(S, S.pp); break;
+    case 16: persist_plan<16>(S, S.pp); break;
+    default: persist_plan<4>(S, S.pp); break;
   }
   const PersistPlan &L = S.pp;
   CgParams &h = *S.h_params;
@@ -3735,7 +3751,7 @@ int solve_fp64(Solver &S, int *Iarray, double *Rarray, int *iter, double *resid,
   }
   const auto choose_apply = [&] {
     S.apply_one = !persist() && !learned && !record && method != 1 && !lowp && iterPREmax > 0 && apply_rule(S);
-    if (S.apply_one) persist_plan<4>(S);
+    if (S.apply_one) persist_plan<4>(S, S.ap, true);
   };
   choose_apply();
   struct ApplyScope {
@@ -3814,10 +3830,10 @@ int solve_fp64(Solver &S, int *Iarray, double *Rarray, int *iter, double *resid,
     S.bnrm2 = dot_device(S, S.b.p, S.b.p);
   }
   if (S.apply_one) {
-    H33_CUDA(cudaMemcpyAsync(S.h_gave_up, S.pp.bar.p + 5, sizeof(unsigned), cudaMemcpyDeviceToHost, S.stream));
+    H33_CUDA(cudaMemcpyAsync(S.h_gave_up, S.ap.bar.p + 1, sizeof(unsigned), cudaMemcpyDeviceToHost, S.stream));
     S.sync();
     if (*S.h_gave_up) {
-      S.pp.bar.zero(S.stream);
+      S.ap.bar.zero(S.stream);
       throw Failure(HECMW33_ERR_TIMEOUT, "a wait of the SSOR application gave up (internal error)");
     }
   }
@@ -4300,8 +4316,8 @@ void launch_mr_persist(Solver &S, const MrPersistArgs &a) {
   H33_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(MrShared))));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(unsigned(S.nsm), 1, 1);
-  cfg.blockDim = dim3(kMrThreads, 1, 1);
-  cfg.dynamicSmemBytes = sizeof(MrShared);
+  cfg.blockDim = dim3(unsigned(32 * S.mpp.warps), 1, 1);
+  cfg.dynamicSmemBytes = offsetof(MrShared, blk) + 2 * size_t(S.mpp.warps) * sizeof(MrShared::blk[0]);
   cfg.stream = S.stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeCooperative;
@@ -4317,6 +4333,15 @@ void run_mr_persist(Solver &S, int nrhs) {
   const size_t n48 = size_t(S.N) * kRhsStride;
   if (L.generation != P.generation) {
     L.rows.upload(P.lo.group_rows, S.stream);
+    // 8 warps a CTA while these have two rows each in the largest colour, else 16: two
+    // handles' solves then fit the SMs together.  ms for one solve / for four handles at
+    // once, 8 load cases, with 16 warps and with 8: 378 nodes 7.3 / 30 and 7.4 / 15.8, 19
+    // thousand 77 / 356 and 83 / 204 (as colour launches 10.3 / 11.9, 103 / 222); with 4
+    // warps 7.7 / 8.8 and 85 / 237.
+    int most = 0;
+    for (size_t g = 0; g + 1 < P.lo.group_rows.size(); g++)
+      most = std::max(most, P.lo.group_rows[g + 1] - P.lo.group_rows[g]);
+    L.warps = most <= 2 * 8 * S.nsm ? 8 : kMrWarps;
     L.lo_gs.upload(P.lo.group_slice, S.stream);
     L.up_gs.upload(P.up.group_slice, S.stream);
     L.iperm.alloc(size_t(S.N));

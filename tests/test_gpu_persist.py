@@ -348,3 +348,48 @@ def test_a_solve_does_not_depend_on_what_the_handle_solved_before(box, precond):
     assert same(mixed[0], cg[0]) and same(mixed[1], bicg[0]) and same(mixed[2], cg[0])
     assert same(mixed[3], bicg[1])
     assert same(back[0], bicg[0]) and same(back[1], cg[1])
+
+
+@pytest.mark.parametrize("call", ["bicgstab", "gmres", "load cases"])
+def test_handles_of_several_threads_beside_each_other(call):
+    """One-launch SSOR applications and load-case solves of three handles at once, with CTAs
+    of the fewest warps (two can share an SM) and of the most."""
+    import threading
+    boxes = [(6, 5, 8), (14, 14, 20), (48, 46, 47)]
+    systems, alone, got, errors = [], [], [None] * 3, []
+
+    def solve(s, m):
+        if call == "load cases":
+            X = np.zeros((3, 3 * m.N))
+            s.set_matrix(m)
+            s.solve_multi(np.stack([m.B, 2.0 * m.B[::-1], m.B * m.B]), X, m.Iarray.copy(), m.Rarray)
+            return X
+        g = m.copy()
+        s.solve(g)
+        return g.X
+
+    for b in boxes:
+        m = box_system(*b)
+        m.set_iter(12)
+        if call != "load cases":
+            m.set_method(2 if call == "bicgstab" else 3)
+        systems.append(m)
+        with GpuSolver() as s:
+            alone.append(solve(s, m))
+
+    def run(k):
+        try:
+            with GpuSolver() as s:
+                for _ in range(4):
+                    got[k] = solve(s, systems[k])
+        except Exception as e:  # noqa: BLE001 -- reported below
+            errors.append(e)
+
+    threads = [threading.Thread(target=run, args=(k,)) for k in range(3)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors
+    for k in range(3):
+        assert np.array_equal(got[k], alone[k])
