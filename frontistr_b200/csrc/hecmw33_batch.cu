@@ -423,13 +423,18 @@ std::string cache_path() {
   return std::string(home ? home : ".") + "/.cache/frontistr_b200_autotune.jsonl";
 }
 
+// Whether the batch's solves run the fused iteration, given four lanes per row or more: the
+// sweeps hold A's own values (matrix and preconditioner change together in a batch).
+bool fusable(const Batch &B, int iterpremax) { return B.kind == 1 && iterpremax == 1 && B.sigma == 1.0; }
+
 std::string batch_key(const Batch &B, int iterpremax) {
-  // the schedule depends on the device, the system sizes and the preconditioner
+  // the schedule depends on the device, the system sizes, the preconditioner and the
+  // iteration's kernel: one tuned for the sweeps with a product is not the fused one's
   uint64_t h = 1469598103934665603ull;
   for (int v : B.node0) h = (h ^ uint64_t(v)) * 1099511628211ull;
   char buf[256];
-  std::snprintf(buf, sizeof(buf), "batch:sm%d:n%d:nz%d:sys%d:pc%d:pre%d:%016llx", B.nsm, B.N, B.N + B.NPL + B.NPU,
-                B.nsys, B.kind, iterpremax, (unsigned long long)h);
+  std::snprintf(buf, sizeof(buf), "batch:sm%d:n%d:nz%d:sys%d:pc%d:pre%d:%016llx%s", B.nsm, B.N, B.N + B.NPL + B.NPU,
+                B.nsys, B.kind, iterpremax, (unsigned long long)h, fusable(B, iterpremax) ? ":fused" : "");
   return buf;
 }
 
@@ -543,8 +548,7 @@ float run_batch(Batch &B, const Schedule &sc, int iterpremax, double tol, int ma
   for (int s = 0; s < B.nsys; s++) B.sys_h[s].skip = (B.zero_diag[s] && iterpremax > 0) ? 1 : 0;
   B.sys_d.upload(B.sys_h, B.stream);
   make_queues(B, sc);
-  // the sweeps hold A's own values in a batch: matrix and preconditioner change together
-  const bool fused = B.kind == 1 && iterpremax == 1 && B.sigma == 1.0 && B.lanes_built >= 4;
+  const bool fused = fusable(B, iterpremax) && B.lanes_built >= 4;
   const int grid = batch_grid(B, fused, sc.cluster);
   BatchArgs a;
   a.A = B.A.view();

@@ -4,6 +4,8 @@ oracle's own hecmw_solve of that system alone, with the drop-in's parity bars
 tolerance), under every launch schedule the autotuner can pick (single CTAs,
 cluster teams of 2 / 4 / 8 CTAs, 4 / 8 / 16 lanes per sweep row), plus the per-system
 codes: 2002 (zero load), 2001 (zero diagonal, not solved), 3001 (MAXIT)."""
+import json
+
 import numpy as np
 import pytest
 
@@ -207,3 +209,32 @@ def test_batch_system_that_diverges_leaves_the_others_alone(monkeypatch):
         x = X[3 * sys_ptr[k]:3 * sys_ptr[k + 1]]
         assert rec["errors"][k] == 0 and abs(int(rec["iter"][k]) - refs[k]["iter"]) <= 2
         assert np.linalg.norm(x - refs[k]["X"]) <= 1e-8 * np.linalg.norm(refs[k]["X"])
+
+
+def test_batch_schedules_of_the_two_kernels_are_kept_apart(tmp_path, monkeypatch):
+    """A cached schedule of the sweeps with a product (SIGMA_DIAG != 1; two lanes per row rule
+    the fused kernel out) is not taken for a batch that runs the fused iteration."""
+    cache = tmp_path / "tune.jsonl"
+    monkeypatch.setenv("HECMW33_AUTOTUNE_CACHE", str(cache))
+    monkeypatch.delenv("HECMW33_BATCH_SCHEDULE", raising=False)
+    systems = random_box_batch(5, edge_range=(2, 6), seed=3)
+    big, sys_ptr = stack_systems(systems)
+    ia, ra = flags(big)
+
+    def solve(sigma, tune=False):
+        ra[1] = sigma
+        X = np.zeros(3 * big.N)
+        with BatchSolver() as bs:
+            bs.set_matrix(big, sys_ptr, ia, ra)
+            if tune:
+                bs.autotune(big.B, X, ia, ra)
+            bs.solve(big.B, X, ia, ra)
+            return bs.info()
+
+    solve(1.2, tune=True)
+    entry = json.loads(cache.read_text().splitlines()[-1])
+    entry["lanes"] = 2
+    cache.write_text(json.dumps(entry) + "\n")
+    unfused, fused = solve(1.2), solve(1.0)
+    assert unfused["tuned"] == 1 and unfused["lanes"] == 2
+    assert fused["tuned"] == 0 and fused["lanes"] >= 4
