@@ -286,6 +286,10 @@ void build_precond_layout(Batch &B, int lanes) {
   B.sync();
 }
 
+// Whether the batch's solves run the fused iteration, given four lanes per row or more: the
+// sweeps hold A's own values (matrix and preconditioner change together in a batch).
+bool fusable(const Batch &B, int iterpremax) { return B.kind == 1 && iterpremax == 1 && B.sigma == 1.0; }
+
 // The schedule before any tuning: every system to a team of C CTAs, C by the larger of
 // the largest system's time on its team and the whole batch's over the resident teams,
 // with a system's time as nodes / C + 230 (the part that more CTAs do not shorten, in
@@ -294,7 +298,14 @@ void build_precond_layout(Batch &B, int lanes) {
 // 34.4, 6 of 4-14 29.8 / 20.4 / 15.3 / 11.5, 128 of 4-14 42.4 / 28.5 / 21.9 / 36.3, 100 of
 // 12-24 422 / 227 / 133 / 128 (four lanes: C = 4 105, C = 8 115); the fixed choice before,
 // teams of 4 for the largest 15 %, took 72.6, 22.8, 23.9 and 250.
-Schedule default_schedule(const Batch &B) {
+// That is the fused iteration, two CTAs an SM.  The unfused one (four an SM: DIAG, SIGMA_DIAG
+// != 1, no preconditioner) gains by large teams too, by C = 1 only while the systems are
+// tiny, and between the two keeps the fixed choice.  ms with the fixed choice / the rule's
+// C, DIAG and SIGMA_DIAG 1.2: 64 of 4-20 C = 8 116 / 43, 159 / 84; 128 of 4-14 C = 4 39 / 24,
+// 57 / 50; 180 of 5-12 C = 4 27 / 19, 40 / 36; 200 of 4-10 C = 2 13.3 / 16.2, 23.0 / 30.1; 400
+// of 4-8 C = 1 7.8 / 12.2, 17.8 / 23.4; 250 of 5-6 (277 nodes in the mean) C = 1 4.65 / 5.66,
+// 13.1 / 11.6; 1000 of 3-6 (168 nodes) C = 1 7.0 / 5.6, 18.0 / 10.6.
+Schedule default_schedule(const Batch &B, bool fused) {
   const double slots = 2.0 * B.nsm, mean = double(B.N) / B.nsys;
   double largest = 0.0, best = 0.0;
   for (int s = 0; s < B.nsys; s++) largest = std::max(largest, double(B.node0[size_t(s) + 1] - B.node0[size_t(s)]));
@@ -306,6 +317,7 @@ Schedule default_schedule(const Batch &B) {
       sc.cluster = c;
     }
   }
+  if (!fused && sc.cluster <= 2 && (sc.cluster == 2 || mean >= 200.0)) return Schedule{8, 4, 0.15};
   sc.lanes = mean > 4096.0 ? 4 : 8;
   sc.big_frac = sc.cluster > 1 ? 1.0 : 0.0;
   return sc;
@@ -400,7 +412,7 @@ void batch_set_matrix(Batch &B, int nsys, const int *sys_ptr, int N, int NP, int
       for (int j = 0; j < 3; j++)
         if (std::fabs(D[9 * size_t(i) + 4 * j]) == 0.0) B.zero_diag[s] = 1;
   if (symbolic) {
-    if (!B.tuned) B.sched = default_schedule(B);
+    if (!B.tuned) B.sched = default_schedule(B, fusable(B, Iarray[4]));
     build_precond_layout(B, B.sched.lanes);
   } else {
     // values only: repack the sweep layouts and refactor the diagonal blocks
@@ -422,10 +434,6 @@ std::string cache_path() {
   const char *home = std::getenv("HOME");
   return std::string(home ? home : ".") + "/.cache/frontistr_b200_autotune.jsonl";
 }
-
-// Whether the batch's solves run the fused iteration, given four lanes per row or more: the
-// sweeps hold A's own values (matrix and preconditioner change together in a batch).
-bool fusable(const Batch &B, int iterpremax) { return B.kind == 1 && iterpremax == 1 && B.sigma == 1.0; }
 
 std::string batch_key(const Batch &B, int iterpremax) {
   // the schedule depends on the device, the system sizes, the preconditioner and the

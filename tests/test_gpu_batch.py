@@ -238,3 +238,28 @@ def test_batch_schedules_of_the_two_kernels_are_kept_apart(tmp_path, monkeypatch
     unfused, fused = solve(1.2), solve(1.0)
     assert unfused["tuned"] == 1 and unfused["lanes"] == 2
     assert fused["tuned"] == 0 and fused["lanes"] >= 4
+
+
+@pytest.mark.parametrize("edge,count,precond,expected", [
+    (5, 300, 3, (4, 0.15)), (5, 300, 1, None),  # 216 nodes each
+    (4, 300, 3, (1, 0.0)),                      # 125 nodes each
+    (12, 8, 3, (8, 1.0)), (12, 8, 1, (8, 1.0)),
+])
+def test_batch_untuned_schedule(edge, count, precond, expected, monkeypatch, tmp_path):
+    """The schedule before any tuning: the unfused iteration keeps teams of 4 for the largest
+    15 % of many mid-sized systems, where single CTAs or teams of 2 are slower."""
+    monkeypatch.setenv("HECMW33_AUTOTUNE_CACHE", str(tmp_path / "none.jsonl"))
+    monkeypatch.delenv("HECMW33_BATCH_SCHEDULE", raising=False)
+    one = random_box_batch(1, edge_range=(edge, edge), seed=2)[0]
+    big, sys_ptr = stack_systems([one] * count)
+    ia, ra = flags(big, precond=precond)
+    X = np.zeros(3 * big.N)
+    with BatchSolver() as bs:
+        bs.set_matrix(big, sys_ptr, ia, ra)
+        rec = bs.solve(big.B, X, ia, ra)
+        info = bs.info()
+    assert not rec["errors"].any()
+    if expected is None:
+        assert info["cluster"] <= 2 and info["big_frac"] in (0.0, 1.0)
+    else:
+        assert (info["cluster"], info["big_frac"]) == expected
