@@ -43,3 +43,49 @@ def test_stream_mode_matches_graph_mode(monkeypatch):
         ib = s.solve(b)
     assert ia["iter"] == ib["iter"]
     assert np.array_equal(a.X, b.X)
+
+
+ROUTES = {  # what is not one launch, so that the two modes differ
+    "DIAG": lambda m: m.set_precond(3),
+    "SIGMA_DIAG": lambda m: m.set_sigma_diag(1.2),
+    "two passes": lambda m: m.set_iterpremax(2),
+    "BF16 SSOR": lambda m: (m.set_sigma_diag(1.2), m.Iarray.__setitem__(41, 1)),
+    "BiCGSTAB": lambda m: m.set_method(2),
+    "BiCGSTAB + ILU": lambda m: (m.set_method(2), m.set_precond(10)),
+}
+
+
+@pytest.mark.parametrize("route", list(ROUTES))
+def test_stream_mode_matches_graph_mode_where_there_is_a_loop(route, monkeypatch):
+    """test_stream_mode_matches_graph_mode's solve is one launch in either mode; these have a
+    loop of launches, captured in a graph or issued kStreamChunk iterations at a time."""
+    m = box_system(12, 10, 20, jitter=0.1, seed=5)
+    m.set_iter(20000)
+    ROUTES[route](m)
+    out = []
+    for graph in ("1", "0"):
+        monkeypatch.setenv("HECMW33_GRAPH", graph)
+        g = m.copy()
+        with GpuSolver() as s:
+            rec = s.solve(g)
+            out.append((rec["iter"], rec["error"], s.last_solve_info()["kernels"], g.X))
+    assert out[0][1] == out[1][1] == 0 and out[0][0] == out[1][0]
+    assert out[0][2] > out[0][0]  # a launch per iteration at least (counted in a graph only)
+    assert np.array_equal(out[0][3], out[1][3])
+
+
+def test_stream_mode_matches_graph_mode_load_cases(monkeypatch):
+    """The load-case loop with SIGMA_DIAG != 1, which is not the one-launch kernel's."""
+    m = box_system(12, 10, 20, jitter=0.1, seed=5)
+    m.set_iter(20000)
+    m.set_sigma_diag(1.2)
+    B = np.stack([m.B, -0.5 * m.B, np.roll(m.B, 3)])
+    out = []
+    for graph in ("1", "0"):
+        monkeypatch.setenv("HECMW33_GRAPH", graph)
+        X = np.zeros_like(B)
+        with GpuSolver() as s:
+            s.set_matrix(m)
+            rec = s.solve_multi(B, X, m.Iarray.copy(), m.Rarray)
+        out.append((rec["iter"], X))
+    assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])

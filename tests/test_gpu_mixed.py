@@ -80,3 +80,38 @@ def test_mixed_zero_rhs_and_maxit():
         info = s.solve(t)
         assert info["error"] == 3001
         assert t.get_flag_converged() == 0
+
+
+@pytest.mark.parametrize("route", ["SSOR, SIGMA_DIAG", "SSOR, two passes", "SSOR, recycled", "ILU, two passes"])
+def test_mode1_where_the_factors_are_bf16(route):
+    """Precision mode 1 on the CG loops that keep BF16 factors (plain CG + SSOR and CG + block
+    ILU run their FP64 one-launch kernels in mode 1 too): other bits than mode 0, the launches
+    of a loop, the FP64 solve's iterations within 2 %, the tolerance on b - A x."""
+    m = box_system(12, 12, 40)
+    m.set_iter(20000)
+    if "SIGMA" in route:
+        m.set_sigma_diag(1.2)
+    if "passes" in route:
+        m.set_iterpremax(2)
+    if "ILU" in route:
+        m.set_precond(10)
+    out = []
+    for mode in (0, 1):
+        g = m.copy()
+        with GpuSolver() as s:
+            if "recycled" in route:
+                s.solve(g)
+                for a in (g.D, g.AL, g.AU):
+                    a *= 1.1
+                g.X[:] = 0.0
+                g.Iarray[96] = 1  # new values, recycled preconditioner
+            g.Iarray[41] = mode
+            rec = s.solve(g)
+            out.append((rec, s.last_solve_info(), g))
+    (ref, _, a), (rec, info, b) = out
+    assert rec["error"] == ref["error"] == 0
+    assert info["kernels"] > 4 * rec["iter"] and not np.array_equal(a.X, b.X)
+    assert rec["iter"] <= 1.02 * ref["iter"] + 1
+    r = b.B - b.to_scipy() @ b.X
+    assert np.linalg.norm(r) <= 1e-8 * np.linalg.norm(b.B)
+    assert np.linalg.norm(b.X - a.X) <= 1e-6 * np.linalg.norm(a.X)

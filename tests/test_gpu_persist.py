@@ -393,3 +393,25 @@ def test_handles_of_several_threads_beside_each_other(call):
     assert not errors
     for k in range(3):
         assert np.array_equal(got[k], alone[k])
+
+
+@pytest.mark.parametrize("method", [2, 3, 4, 5, 6, 7])
+@pytest.mark.parametrize("name", ["box_2x1x3", "hubs", "grid16_14x14x20", "box_48x46x47"])
+def test_one_launch_application_is_bitwise_the_colour_launches(name, method, monkeypatch):
+    """ssor_apply_persist_kernel, with 4 warps a CTA and with 16, against a launch per colour:
+    the same arithmetic in the same order, so the same bits after any iterations."""
+    if name == "box_48x46x47" and method > 3:
+        pytest.skip("the kernel's shape is the same for every method")
+    m = box_system(48, 46, 47) if name == "box_48x46x47" else SYSTEMS[name]()
+    m.set_iter(25)
+    m.set_method(method)
+    out = []
+    for launches in ("0", "1"):
+        monkeypatch.setenv("HECMW33_APPLY_LAUNCHES", launches)
+        g = m.copy()
+        with GpuSolver() as s:
+            rec = s.solve(g)
+            out.append((rec["iter"], rec["error"], g.X, s.last_solve_info()["kernels"]))
+    assert out[0][:2] == out[1][:2] and np.array_equal(out[0][2], out[1][2])
+    if method == 2:  # whose count has the launches inside the graph
+        assert out[0][3] < out[1][3]
