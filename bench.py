@@ -602,12 +602,16 @@ def bench_learned_newton(args):
                        for x in steps], "systems": rows, "wall_s": wall}
 
 
-def iteration_bytes(n, nz):
+def iteration_bytes(n, nz, fused=False):
     """Algorithmic bytes of one FP64 CG+SSOR iteration on a one-domain system of n block
     rows and nz blocks: the reference's SpMV model (hecmw_solver_Iterative.f90:211-217),
     one SSOR application (off-diagonal blocks with their columns, the diagonal LU read
-    by both sweeps, row pointers, vectors) and the minimum fused vector traffic."""
+    by both sweeps, row pointers, vectors) and the minimum fused vector traffic.
+    fused: the iteration without a product (h33_persist.cuh): each off-diagonal block and
+    column once, the diagonal LU twice, the vector passes of its two sweeps and its update."""
     off = nz - n
+    if fused:
+        return 76 * off + 2 * 72 * n + (4 + 11 + 9) * 24 * n
     spmv = 72 * nz + 4 * off + 8 * (n + 1) + 24 * n + 24 * n
     ssor = 76 * off + 2 * 72 * n + 2 * 8 * (n + 1) + 4 * 24 * n
     vec = 10 * 24 * n
@@ -665,10 +669,10 @@ def bench_batched(args):
             g.Iarray[96] = g.Iarray[97] = 0
             r1 = s.solve_resident(g.B, g.X, g.Iarray, g.Rarray)
             t_seq += r1["t_solve"]
-    # algorithmic bytes of the batch: every system's CG+SSOR iterations times its
-    # per-iteration bytes (the reference's SpMV model plus the SSOR and vector terms)
+    # algorithmic bytes of the batch: every system's CG+SSOR iterations times the
+    # per-iteration bytes of the kernel that ran (fused with four lanes per row or more)
     its = np.asarray(rec["iter"], dtype=np.float64)
-    nbytes = float(sum(it * iteration_bytes(mk.N, mk.NZ) for it, mk in zip(its, systems)))
+    nbytes = float(sum(it * iteration_bytes(mk.N, mk.NZ, info["lanes"] >= 4) for it, mk in zip(its, systems)))
     peak, peak_kind = measured_peaks()
     out["roofline"] = {"bound": "hbm", "kernel": "batch_cg_kernel (the whole batched solve, one launch)",
                        "algorithmic_bytes": nbytes, "achieved": nbytes / t_b / 1e9, "peak": peak,

@@ -879,7 +879,9 @@ HECMW33_API void hecmw33_gpu_batch_info(const int *handle, int *info, double *di
   dinfo[0] = B.last_ms * 1e-3;
   dinfo[1] = B.last_setup_s;
   dinfo[2] = B.sched.big_frac;
-  const size_t held = B.raw.bytes() + B.alu.bytes() + B.A.bytes() + B.lo.bytes() + B.up.bytes() + 6 * B.b.bytes();
+  const size_t held = B.raw.bytes() + B.alu.bytes() + B.A.bytes() + B.lo.bytes() + B.up.bytes() + 6 * B.b.bytes() +
+                      B.zu.bytes() + B.g.bytes() + B.h.bytes() + B.px.bytes() + B.pl.bytes() + B.iperm.bytes() +
+                      B.lo_desc.bytes() + B.up_desc.bytes();
   dinfo[3] = double(held);
   HB_END
 }

@@ -559,6 +559,7 @@ struct Solver {
   int build_counter = 0;  // monotonic id of preconditioner builds (graph cache key)
   // last-solve record
   int last_iter = 0, last_outer = 0, last_kernels = 0, last_learned = 0, last_fallback = 0;
+  bool last_fused = false;  // the last solve was cg_ssor_persist_kernel's: no product
   double last_solve_s = 0.0, last_setup_s = 0.0, last_true_resid = 0.0;
 
   Solver() {
@@ -2117,6 +2118,7 @@ float run_cg_persist(Solver &S, double tol, int maxit, int *kernels) {
     default: launch_persist<4>(S, a); break;
   }
   H33_CUDA(cudaEventRecord(S.ev1, S.stream));
+  S.last_fused = P.kind == 1;
   H33_CUDA(cudaMemcpyAsync(S.h_state, S.state.p, sizeof(CgState), cudaMemcpyDeviceToHost, S.stream));
   // whichever CTA gave up: the one that writes the state may have passed every barrier
   H33_CUDA(cudaMemcpyAsync(S.h_gave_up, L.bar.p + 1, sizeof(unsigned), cudaMemcpyDeviceToHost, S.stream));
@@ -3033,6 +3035,7 @@ void assemble_hex8(Solver &S, int n_node, const double *coords, int n_elem, cons
 }
 
 int prepare_solve(Solver &S, int *Iarray, double *Rarray, double *sigma, bool *auto_sigma) {
+  S.last_fused = false;
   if (!S.has_matrix) throw Failure(HECMW33_ERR_NO_MATRIX, "no matrix: call hecmw33_gpu_set_matrix first");
   // zero right-hand side (hecmw_solver.f90:32-37; hecmw_solver_Iterative.f90:284-323,
   // with the MPC constants)
@@ -3819,6 +3822,7 @@ int solve_fp64(Solver &S, int *Iarray, double *Rarray, int *iter, double *resid,
         if (auto_sigma) sigma = 1.0;
         method = METHOD2;
         learned = 0;
+        S.last_fused = false;
         relane(S, false);
         if (lowp) ensure_lowp(S);
         choose_apply();
@@ -5355,12 +5359,23 @@ HECMW33_API void hecmw33_gpu_last_solve_info(const int *handle, int *info, doubl
                         2.0 * 2.0 * 24.0 * N;
   const double vec = 10.0 * 24.0 * N;
   dinfo[2] = spmv;
-  dinfo[3] = spmv + sweeps + vec;
+  // the fused iteration (h33_persist.cuh) has no product and reads each off-diagonal block
+  // once; of vectors the backward sweep reads g and r and writes z and v, the forward one
+  // reads v, g, z, p, q, h and pl (half a vector) and writes u, p, q, h and pl, the update
+  // reads and writes x, r and g and reads p, q and h
+  const double fused = 76.0 * (NPL + NPU) + 2.0 * 72.0 * N + (4.0 + 11.0 + 9.0) * 24.0 * N;
+  dinfo[3] = S.last_fused ? fused : spmv + sweeps + vec;
   size_t held = S.raw.bytes() + S.A.bytes() + S.pc.lo.bytes() + S.pc.up.bytes() + S.pc.alu_fwd.bytes() +
                 S.pc.alu_bwd.bytes() + S.pc.ilu_raw.bytes();
   for (auto *v : {&S.b, &S.x, &S.r, &S.z, &S.p, &S.q, &S.w, &S.zp}) held += v->bytes();
   held += S.pc.alu32_fwd.bytes() + S.pc.alu32_bwd.bytes();
   for (auto *v : {&S.bf, &S.xf, &S.rf, &S.zf, &S.pf, &S.qf, &S.wf, &S.zpf}) held += v->bytes();
+  for (const PersistPlan *L : {&S.pp, &S.ap})
+    held += L->lo_items.bytes() + L->up_items.bytes() + L->iperm.bytes() + L->zu.bytes() + L->pl.bytes() +
+            L->parts.bytes() + L->bar.bytes();
+  const MrPersistPlan &M = S.mpp;
+  held += M.rows.bytes() + M.lo_gs.bytes() + M.up_gs.bytes() + M.iperm.bytes() + M.z.bytes() + M.u.bytes() +
+          M.pl.bytes() + M.parts.bytes() + M.bar.bytes();
   dinfo[4] = double(held);
   dinfo[5] = S.last_true_resid;
   H33_ENTRY_END

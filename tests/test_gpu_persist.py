@@ -415,3 +415,27 @@ def test_one_launch_application_is_bitwise_the_colour_launches(name, method, mon
     assert out[0][:2] == out[1][:2] and np.array_equal(out[0][2], out[1][2])
     if method == 2:  # whose count has the launches inside the graph
         assert out[0][3] < out[1][3]
+
+
+def test_reported_bytes_are_those_of_the_kernel_that_ran():
+    """The fused iteration has no product, and its plans' buffers count as held."""
+    m = box_system(14, 14, 20)
+    m.set_iter(20000)
+    off = m.NPL + m.NPU
+    with GpuSolver() as s:
+        s.set_matrix(m)
+        X = np.zeros(3 * m.N)
+        ia, ra = m.Iarray.copy(), m.Rarray.copy()
+        ia[4] = 2  # two passes: a loop of launches
+        s.solve_resident(m.B, X, ia, ra)
+        launches = s.last_solve_info()
+        X[:] = 0.0
+        s.solve_resident(m.B, X, m.Iarray, m.Rarray)
+        fused = s.last_solve_info()
+        s.solve_multi(np.stack([m.B, m.B]), np.zeros((2, 3 * m.N)), m.Iarray, m.Rarray)
+        cases = s.last_solve_info()
+    assert launches["iter_bytes"] > launches["spmv_bytes"] + 76 * off
+    assert fused["iter_bytes"] == 76 * off + 144 * m.N + 24 * 24 * m.N
+    # z with u or v 48, the direction's rest 12, the inverse permutation 4 bytes a node
+    assert fused["device_bytes"] - launches["device_bytes"] >= 64 * m.N
+    assert cases["device_bytes"] - fused["device_bytes"] >= (2 * 8 + 4) * 48 * m.N  # 48 numbers a node
