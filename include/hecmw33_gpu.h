@@ -48,7 +48,8 @@
  *                       stay FP64, so the convergence test is the reference's.  CG with
  *                       an SSOR of the current values (one pass, SIGMA_DIAG = 1) runs as
  *                       in mode 0: it reads each FP64 block once per iteration, fewer
- *                       bytes than BF16 sweeps beside an FP64 product
+ *                       bytes than BF16 sweeps beside an FP64 product.  So does CG with
+ *                       block ILU (one pass): one launch for all levels is the faster
  *                  = 2  mixed precision, restarted refinement: inner FP32 CG (FP32
  *                       matrix and preconditioner copies, FP64 dot products) from zero
  *                       to Rarray(42) relative (0 -> 1e-4), FP64 correction and true
@@ -338,7 +339,8 @@ HECMW33_API void hecmw33_gpu_learn_eval(const int *handle, const float *theta, c
  *   steps (1 for the FP64 solve);
  *   dinfo[0] solve seconds (device events), dinfo[1] setup seconds,
  *   dinfo[2] algorithmic SpMV bytes (reference model: 72 NZ + 4 (NPL+NPU)
- *   + 8 (N+1) + 24 N + 24 NP), dinfo[3] algorithmic bytes of one FP64 iteration,
+ *   + 8 (N+1) + 24 N + 24 NP), dinfo[3] algorithmic bytes of one FP64 iteration (of
+ *   the fused one, which has no product, where that ran),
  *   dinfo[4] device bytes held by the handle, dinfo[5] final FP64 true relative
  *   residual ||b - A x|| / ||b||;
  *   info[8] learned preconditioner used (1/0), info[9] iteration at which its
