@@ -51,15 +51,16 @@ struct MrShared {
   double2 blk[2 * kMrWarps][16 * kMrBlock];  // last: as many as the CTA has half-warps
 };
 
-__device__ __forceinline__ void mr_persist_barrier(const MrPersistArgs &a, MrShared &sh, unsigned &target) {
-  target += gridDim.x;
+__device__ __forceinline__ void mr_persist_barrier(const MrPersistArgs &a, MrShared &sh, GridWay &way) {
+  way.target += gridDim.x;
+  way.gone = sh.dead;  // as in the single application
   __syncthreads();
-  if (threadIdx.x == 0) grid_meet(a.bar, target, a.polls, sh.dead);
+  if (threadIdx.x == 0) grid_meet(a.bar, way, a.polls, sh.dead);
   __syncthreads();
 }
 
 // Sum over the grid for every load case, in sh.res; includes a barrier.
-__device__ __forceinline__ void mr_persist_sum(const MrPersistArgs &a, MrShared &sh, unsigned &target, double v,
+__device__ __forceinline__ void mr_persist_sum(const MrPersistArgs &a, MrShared &sh, GridWay &way, double v,
                                                int slot) {
   const int l = threadIdx.x & 15, hw = threadIdx.x >> 4, nh = blockDim.x >> 4;
   double *parts = a.parts + size_t(slot) * gridDim.x * kMaxRhs;
@@ -70,7 +71,7 @@ __device__ __forceinline__ void mr_persist_sum(const MrPersistArgs &a, MrShared 
     for (int k = 0; k < nh; k++) s += sh.red[k][threadIdx.x];
     parts[size_t(blockIdx.x) * kMaxRhs + threadIdx.x] = s;
   }
-  mr_persist_barrier(a, sh, target);
+  mr_persist_barrier(a, sh, way);
   double s = 0.0;
   for (int i = hw; i < int(gridDim.x); i += nh) s += __ldcg(parts + size_t(i) * kMaxRhs + l);
   sh.red[hw][l] = s;
@@ -134,7 +135,7 @@ __device__ __forceinline__ void mr_persist_row(const SellView<double> &A, int s,
 // One sweep: MODE 0 backward, 1 forward on the direction, 2 forward from r for the load
 // cases of sh.again (start and refresh; the others keep g).
 template <int K, int MODE>
-__device__ __forceinline__ double mr_persist_sweep(const MrPersistArgs &a, MrShared &sh, unsigned &target) {
+__device__ __forceinline__ double mr_persist_sweep(const MrPersistArgs &a, MrShared &sh, GridWay &way) {
   constexpr int RPS = 32 / K;
   const int lane = threadIdx.x & 15, hwl = threadIdx.x >> 4;
   const int hw = hwl * gridDim.x + blockIdx.x, nhw = (blockDim.x >> 4) * gridDim.x;
@@ -150,7 +151,7 @@ __device__ __forceinline__ double mr_persist_sweep(const MrPersistArgs &a, MrSha
     const int r0 = __ldg(a.rows + g), r1 = __ldg(a.rows + g + 1), s0 = __ldg(gs + g);
     int row = r0 + hw, s = s0 + (row - r0) / RPS, roff = (row - r0) % RPS;
     int len = row < r1 ? __ldg(L.rowlen + s * 32 + roff) : 0;
-    if (c) mr_persist_barrier(a, sh, target);
+    if (c) mr_persist_barrier(a, sh, way);
     while (row < r1) {
       const double *lu = a.alu + row;
       const double a0 = __ldg(lu), a1 = __ldg(lu + n), a2 = __ldg(lu + 2 * n);
@@ -247,7 +248,7 @@ __global__ void __launch_bounds__(kMrThreads, 1) mr_cg_persist_kernel(const MrPe
   MrShared &sh = *reinterpret_cast<MrShared *>(mr_smem);
   const int tid = threadIdx.x, lane = tid & 15;
   const int hw = (tid >> 4) * gridDim.x + blockIdx.x, nhw = (blockDim.x >> 4) * gridDim.x;
-  unsigned target = 0;
+  GridWay way;
   if (tid < kMaxRhs) {
     CgState s = {};
     s.tol = a.prm->tol;
@@ -287,7 +288,7 @@ __global__ void __launch_bounds__(kMrThreads, 1) mr_cg_persist_kernel(const MrPe
     }
     __syncthreads();
   };
-  mr_persist_sum(a, sh, target, mr_persist_resid<true>(a, sh, true), 0);
+  mr_persist_sum(a, sh, way, mr_persist_resid<true>(a, sh, true), 0);
   if (tid < kMaxRhs) {
     CgState &s = sh.st[tid];
     s.bnrm2 = sh.res[tid];
@@ -306,18 +307,18 @@ __global__ void __launch_bounds__(kMrThreads, 1) mr_cg_persist_kernel(const MrPe
   while (sh.any) {
     guard++;
     if (restart) {
-      mr_persist_sweep<K, 2>(a, sh, target);
-      mr_persist_barrier(a, sh, target);
+      mr_persist_sweep<K, 2>(a, sh, way);
+      mr_persist_barrier(a, sh, way);
     }
     if (tid < kMaxRhs) {
       if (!sh.st[tid].done) sh.st[tid].guard++;
       sh.again[tid] = 0;
     }
     __syncthreads();
-    mr_persist_sum(a, sh, target, mr_persist_sweep<K, 0>(a, sh, target), 0);
+    mr_persist_sum(a, sh, way, mr_persist_sweep<K, 0>(a, sh, way), 0);
     if (tid < kMaxRhs && !sh.st[tid].done) fin_rho(&sh.st[tid], sh.res[tid]);
     __syncthreads();
-    mr_persist_sum(a, sh, target, mr_persist_sweep<K, 1>(a, sh, target), 1);
+    mr_persist_sum(a, sh, way, mr_persist_sweep<K, 1>(a, sh, way), 1);
     if (tid < kMaxRhs && !sh.st[tid].done) fin_pq(&sh.st[tid], sh.res[tid]);
     __syncthreads();
     {
@@ -340,7 +341,7 @@ __global__ void __launch_bounds__(kMrThreads, 1) mr_cg_persist_kernel(const MrPe
             }
           }
         }
-      mr_persist_sum(a, sh, target, rr, 2);
+      mr_persist_sum(a, sh, way, rr, 2);
     }
     if (tid < kMaxRhs) {
       CgState &s = sh.st[tid];
@@ -351,8 +352,8 @@ __global__ void __launch_bounds__(kMrThreads, 1) mr_cg_persist_kernel(const MrPe
     restart = false;
     if (need) {  // a true residual is due for some load cases
       nodes_x();
-      mr_persist_barrier(a, sh, target);
-      mr_persist_sum(a, sh, target, mr_persist_resid<false>(a, sh, sh.again[lane] != 0), 1);
+      mr_persist_barrier(a, sh, way);
+      mr_persist_sum(a, sh, way, mr_persist_resid<false>(a, sh, sh.again[lane] != 0), 1);
       if (tid < kMaxRhs && sh.again[tid]) {
         CgState &s = sh.st[tid];
         s.rr = sh.res[tid];

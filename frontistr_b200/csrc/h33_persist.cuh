@@ -125,19 +125,29 @@ struct PersistShared {
   int dead;
 };
 
-// One thread's arrival at the grid barrier and its wait until *bar has reached target;
+// A thread's way through the grid's barriers: the arrivals at the next one, and whether it
+// has given up.  The CG keeps that in a register (read from shared memory it cost 30 ns a
+// barrier, 1 % of the block ILU's levels); in the single application and the load cases,
+// short of registers, reading it is 3 % the faster.
+struct GridWay {
+  unsigned target = 0;
+  bool gone = false;
+};
+
+// One thread's arrival at the grid barrier and its wait until *bar has reached the target;
 // after `polls` polls, or when another CTA has given up, it gives up (dead).  A CTA that
 // has given up arrives nowhere any more, so none passes a barrier that a late one has not
 // reached; the others see its mark in bar[1] and give up too.
-__device__ __forceinline__ void grid_meet(unsigned *bar, unsigned target, int polls, int &dead) {
-  if (dead) return;
+__device__ __forceinline__ void grid_meet(unsigned *bar, GridWay &way, int polls, int &dead) {
+  if (way.gone) return;
   asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
   unsigned v;
   int tries = 0;
   for (;;) {
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
-    if (int(v - target) >= 0) break;
+    if (int(v - way.target) >= 0) break;
     if (++tries > polls || ((tries & 1023) == 0 && *((volatile unsigned *)(bar + 1)))) {
+      way.gone = true;
       dead = 1;
       *((volatile unsigned *)(bar + 1)) = 1u;
       break;
@@ -149,25 +159,25 @@ __device__ __forceinline__ void grid_meet(unsigned *bar, unsigned target, int po
 // cluster and the barrier its hardware barrier; else a counter in global memory, its
 // wait bounded.
 template <bool CLUSTER>
-__device__ __forceinline__ void persist_barrier(const PersistArgs &a, PersistShared &sh, unsigned &target) {
+__device__ __forceinline__ void persist_barrier(const PersistArgs &a, PersistShared &sh, GridWay &way) {
   if constexpr (CLUSTER) {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
   } else {
-    target += gridDim.x;
+    way.target += gridDim.x;
     __syncthreads();
-    if (threadIdx.x == 0) grid_meet(a.bar, target, a.polls, sh.dead);
+    if (threadIdx.x == 0) grid_meet(a.bar, way, a.polls, sh.dead);
     __syncthreads();
   }
 }
 
 // Sum over the grid, the same value in every thread; includes a barrier.
 template <bool CLUSTER>
-__device__ __forceinline__ double persist_sum(const PersistArgs &a, PersistShared &sh, unsigned &target, double v,
+__device__ __forceinline__ double persist_sum(const PersistArgs &a, PersistShared &sh, GridWay &way, double v,
                                               int slot) {
   v = block_sum(v, sh.red);
   double *parts = a.parts + slot * gridDim.x;
   if (threadIdx.x == 0) parts[blockIdx.x] = v;
-  persist_barrier<CLUSTER>(a, sh, target);
+  persist_barrier<CLUSTER>(a, sh, way);
   if (threadIdx.x < 32) {
     double s = 0.0;
     for (int i = threadIdx.x; i < int(gridDim.x); i += 32) s += __ldcg(parts + i);
@@ -411,11 +421,11 @@ __device__ __forceinline__ double ssor_sweep(const SsorVecs &a, const double *va
 }
 
 template <int K, int MODE, bool CLUSTER>
-__device__ __forceinline__ double persist_sweep(const PersistArgs &a, PersistShared &sh, unsigned &target, int w,
+__device__ __forceinline__ double persist_sweep(const PersistArgs &a, PersistShared &sh, GridWay &way, int w,
                                                 double beta, bool first) {
   const PersistSweep S = MODE == 0 ? a.up : a.lo;
   return ssor_sweep<K, MODE, CLUSTER>(a.v, S.val, S.col, ListCursor{S.items + size_t(w) * S.stride, a.ncolor},
-                                      [&] { persist_barrier<CLUSTER>(a, sh, target); }, beta, first);
+                                      [&] { persist_barrier<CLUSTER>(a, sh, way); }, beta, first);
 }
 
 // Descriptors of a layout's slices for GroupCursor.
@@ -539,7 +549,7 @@ __global__ void __launch_bounds__(32 * persist_warps<K>(), 1) cg_ssor_persist_ke
   const int tid = threadIdx.x, warp = tid >> 5;
   const int w = warp * gridDim.x + blockIdx.x;  // this warp's list: neighbouring slices on different SMs
   const int gt = blockIdx.x * blockDim.x + tid, nt = gridDim.x * blockDim.x;
-  unsigned target = 0;
+  GridWay way;
   persist_begin(a, sh);
   // x in position order; z and u start at zero (padding blocks gather position 0)
   for (int i = gt; i < a.n; i += nt) {
@@ -551,23 +561,23 @@ __global__ void __launch_bounds__(32 * persist_warps<K>(), 1) cg_ssor_persist_ke
     }
   }
   CgState &st = sh.st;
-  persist_bnrm(sh, persist_sum<CLUSTER>(a, sh, target, persist_resid<true>(a), 0));
+  persist_bnrm(sh, persist_sum<CLUSTER>(a, sh, way, persist_resid<true>(a), 0));
   const int n3 = 3 * a.n, n2 = n3 / 2;
   bool restart = true;  // g from r
   while (!st.done) {
     if (restart) {
-      persist_sweep<K, 2, CLUSTER>(a, sh, target, w, 0.0, false);
-      persist_barrier<CLUSTER>(a, sh, target);
+      persist_sweep<K, 2, CLUSTER>(a, sh, way, w, 0.0, false);
+      persist_barrier<CLUSTER>(a, sh, way);
       restart = false;
     }
     if (tid == 0) st.guard++;
-    const double rho = persist_sum<CLUSTER>(a, sh, target, persist_sweep<K, 0, CLUSTER>(a, sh, target, w, 0.0, false), 0);
+    const double rho = persist_sum<CLUSTER>(a, sh, way, persist_sweep<K, 0, CLUSTER>(a, sh, way, w, 0.0, false), 0);
     if (tid == 0) fin_rho(&st, rho);
     __syncthreads();
     if (st.done) break;
     const bool first = st.iter == 1;
     const double pq =
-        persist_sum<CLUSTER>(a, sh, target, persist_sweep<K, 1, CLUSTER>(a, sh, target, w, st.beta, first), 1);
+        persist_sum<CLUSTER>(a, sh, way, persist_sweep<K, 1, CLUSTER>(a, sh, way, w, st.beta, first), 1);
     if (tid == 0) fin_pq(&st, pq);
     __syncthreads();
     if (st.done) break;
@@ -607,9 +617,9 @@ __global__ void __launch_bounds__(32 * persist_warps<K>(), 1) cg_ssor_persist_ke
           rr += r * r;
         }
       }
-      if (refresh) persist_barrier<CLUSTER>(a, sh, target);
+      if (refresh) persist_barrier<CLUSTER>(a, sh, way);
       else {
-        rr = persist_sum<CLUSTER>(a, sh, target, rr, 2);
+        rr = persist_sum<CLUSTER>(a, sh, way, rr, 2);
         if (tid == 0) fin_rr(&st, rr);
         __syncthreads();
       }
@@ -620,8 +630,8 @@ __global__ void __launch_bounds__(32 * persist_warps<K>(), 1) cg_ssor_persist_ke
 #pragma unroll
         for (int c = 0; c < 3; c++) a.x[3 * node + c] = __ldcg(a.px + 3 * i + c);
       }
-      persist_barrier<CLUSTER>(a, sh, target);
-      persist_true_resid(sh, persist_sum<CLUSTER>(a, sh, target, persist_resid<false>(a), 2), refresh);
+      persist_barrier<CLUSTER>(a, sh, way);
+      persist_true_resid(sh, persist_sum<CLUSTER>(a, sh, way, persist_resid<false>(a), 2), refresh);
       restart = true;
     }
     persist_ctl(sh);
@@ -637,7 +647,7 @@ __global__ void __launch_bounds__(32 * persist_warps<K>(), 1) cg_ssor_persist_ke
     }
   }
   persist_end(a, sh);
-  if constexpr (CLUSTER) persist_barrier<true>(a, sh, target);
+  if constexpr (CLUSTER) persist_barrier<true>(a, sh, way);
 }
 
 // ---- one application of the SSOR ---------------------------------------------------
@@ -666,12 +676,13 @@ __global__ void __launch_bounds__(32 * persist_warps<K>(), 1) ssor_apply_persist
   const int lane = threadIdx.x & 31, roff = lane / K;
   const bool leader = (lane & (K - 1)) == 0;
   const int w = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
-  unsigned target = 0;
+  GridWay way;
   if (threadIdx.x == 0) dead = 0;
   const auto barrier = [&] {
-    target += gridDim.x;
+    way.target += gridDim.x;
+    way.gone = dead;
     __syncthreads();
-    if (threadIdx.x == 0) grid_meet(a.bar, target, a.polls, dead);
+    if (threadIdx.x == 0) grid_meet(a.bar, way, a.polls, dead);
     __syncthreads();
   };
   {
@@ -752,7 +763,7 @@ __global__ void __launch_bounds__(32 * persist_warps<K>(), 1) ssor_apply_persist
 //
 // One direction: forward z = LU^-1 (r - L z), backward z -= LU^-1 (U z) with RHO = r.z.
 template <int K, bool BACK, bool CLUSTER>
-__device__ __forceinline__ double persist_levels(const PersistArgs &a, PersistShared &sh, unsigned &target, int w) {
+__device__ __forceinline__ double persist_levels(const PersistArgs &a, PersistShared &sh, GridWay &way, int w) {
   constexpr int U = 2;
   const int lane = threadIdx.x & 31;
   const int sub = lane & (K - 1), roff = lane / K;
@@ -770,7 +781,7 @@ __device__ __forceinline__ double persist_levels(const PersistArgs &a, PersistSh
   for (int u = 0; u < U; u++) col[u] = u < it.y ? __ldg(S.col + (it.x + u) * 32 + lane) : 0;
   int node = it.w == kPEnd ? 0 : __ldg(perm + it.z + (roff < (it.w & 63) ? roff : 0));
   for (int c = 0; c < nstep; c++) {
-    if (c) persist_barrier<CLUSTER>(a, sh, target);
+    if (c) persist_barrier<CLUSTER>(a, sh, way);
     while ((it.w >> 6) == c) {
       const bool act = roff < (it.w & 63);
       const int row = it.z + (act ? roff : 0), i3 = 3 * node;
@@ -874,17 +885,17 @@ __global__ void __launch_bounds__(32 * persist_warps<K>(), 1) cg_ilu_persist_ker
   const int tid = threadIdx.x;
   const int w = (tid >> 5) * gridDim.x + blockIdx.x;
   const int gt = blockIdx.x * blockDim.x + tid, nt = gridDim.x * blockDim.x;
-  unsigned target = 0;
+  GridWay way;
   persist_begin(a, sh);
   const int n3 = 3 * a.n;
   for (int i = gt; i < n3; i += nt) a.pz[i] = 0.0;  // padding blocks gather node 0
-  persist_bnrm(sh, persist_sum<CLUSTER>(a, sh, target, persist_resid<true>(a), 0));
+  persist_bnrm(sh, persist_sum<CLUSTER>(a, sh, way, persist_resid<true>(a), 0));
   CgState &st = sh.st;
   while (!st.done) {
     if (tid == 0) st.guard++;
-    persist_levels<K, false, CLUSTER>(a, sh, target, w);
-    persist_barrier<CLUSTER>(a, sh, target);
-    const double rho = persist_sum<CLUSTER>(a, sh, target, persist_levels<K, true, CLUSTER>(a, sh, target, w), 0);
+    persist_levels<K, false, CLUSTER>(a, sh, way, w);
+    persist_barrier<CLUSTER>(a, sh, way);
+    const double rho = persist_sum<CLUSTER>(a, sh, way, persist_levels<K, true, CLUSTER>(a, sh, way, w), 0);
     if (tid == 0) fin_rho(&st, rho);
     __syncthreads();
     if (st.done) break;
@@ -894,8 +905,8 @@ __global__ void __launch_bounds__(32 * persist_warps<K>(), 1) cg_ilu_persist_ker
       const double z = __ldcg(a.pz + i);
       a.pp[i] = first ? z : z + beta * __ldcg(a.pp + i);
     }
-    persist_barrier<CLUSTER>(a, sh, target);
-    const double pq = persist_sum<CLUSTER>(a, sh, target, persist_product(a), 1);
+    persist_barrier<CLUSTER>(a, sh, way);
+    const double pq = persist_sum<CLUSTER>(a, sh, way, persist_product(a), 1);
     if (tid == 0) fin_pq(&st, pq);
     __syncthreads();
     if (st.done) break;
@@ -910,18 +921,18 @@ __global__ void __launch_bounds__(32 * persist_warps<K>(), 1) cg_ilu_persist_ker
         rr += r * r;
       }
     }
-    rr = persist_sum<CLUSTER>(a, sh, target, rr, 2);
+    rr = persist_sum<CLUSTER>(a, sh, way, rr, 2);
     if (!refresh) {
       if (tid == 0) fin_rr(&st, rr);
       __syncthreads();
     }
     if (refresh || st.recompute)
-      persist_true_resid(sh, persist_sum<CLUSTER>(a, sh, target, persist_resid<false>(a), 1), refresh);
+      persist_true_resid(sh, persist_sum<CLUSTER>(a, sh, way, persist_resid<false>(a), 1), refresh);
     // r (and x) are complete at a barrier before the next sweep gathers or overwrites
     persist_ctl(sh);
   }
   persist_end(a, sh);
-  if constexpr (CLUSTER) persist_barrier<true>(a, sh, target);
+  if constexpr (CLUSTER) persist_barrier<true>(a, sh, way);
 }
 
 }  // namespace h33

@@ -1991,8 +1991,8 @@ int persist_grid(Solver &S, bool ilu, int rows) {
 }
 
 // Warps of a CTA of the single application: 4 while these have a slice each in the largest
-// colour, else all 16.  Alone it makes no difference, but four of 4 warps leave room beside
-// them for the launches of other handles; ms for one solve / for four handles at once, with
+// colour, else all 16.  Alone they are 1 % slower, but 4 warps leave room beside them for
+// the launches of other handles; ms for one solve / for four handles at once, with
 // 16 warps and with 4: BiCGSTAB on 378 nodes 9.1 / 31 and 9.2 / 10.7, 19 thousand 106 / 409
 // and 107 / 129, 45 thousand 77 / 318 and 77 / 114 (as colour launches 11.3 / 12.5, 161 /
 // 216, 122 / 182); 118 thousand nodes need 7: 118 / 504 with 16, 119 / 657 with 7.
