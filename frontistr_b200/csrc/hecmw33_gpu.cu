@@ -4432,7 +4432,7 @@ float run_multi_chunk(Solver &S, int nrhs, const double *dB, double *dX, int ite
   H33_CUDA(cudaMemcpyAsync(S.params.p, S.h_params, sizeof(CgParams), cudaMemcpyHostToDevice, s));
   H33_CUDA(cudaEventRecord(S.ev0, s));
   // one launch while a half-warp of its grid has about two rows a colour or fewer: 16
-  // load cases at 7,350 rows a colour 721 us an iteration against 783 as colour launches,
+  // load cases at 7,350 rows a colour 695 us an iteration against 783 as colour launches,
   // at 17 thousand 1521 against 1477
   const bool persist = !learned && S.pc.kind == 1 && persist_ok(S, iterpremax) &&
                        S.N / std::max(S.pc.ncolor, 1) <= 2 * 2 * kMrWarps * S.nsm;
