@@ -1219,7 +1219,7 @@ void relane(Solver &S, bool cg) {
   const int grid = std::max(1, std::min((S.N + kThreads - 1) / kThreads, S.nsm * 8));
   if (P.kind == 1) {
     DevArray<double> raw;
-    raw.alloc(9 * (size_t(S.N) + S.NPL + S.NPU));
+    raw.alloc(S.raw.n);
     for (auto *d : {&P.lo, &P.up})
       if (d->nslots) launch_k(S.stream, unpack_sell_kernel, grid, kThreads, static_cast<const double *>(d->val.p),
                               static_cast<const int *>(d->src.p), d->nslots, raw.p);
