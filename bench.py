@@ -363,8 +363,8 @@ def bench_multi(solver, m, nrhs=16, learned=False):
 def bench_config3(tol=1e-10):
     """Mixed precision on the harder system: 80x80x80 HEX8, interior nodes jittered by
     +-0.2h, log-normal E (median 210000, sigma 1.0), nu uniform in [0.25, 0.40]
-    (seeded), same supports and load; FP64 CG+SSOR and the three mixed modes to 1e-10,
-    each with its error against the FP64 solution."""
+    (seeded), same supports and load; FP64 CG+SSOR and the three mixed modes to 1e-10
+    (mode 1 runs mode 0's one FP64 launch), each with its error against the FP64 solution."""
     import numpy as np
     from frontistr_b200.mesh import box_system
     from frontistr_b200.solver import GpuSolver
@@ -880,7 +880,9 @@ def main():
                 mm.B[3 * node:3 * node + 3] = t
             mm.Iarray[97] = 0
             mm.Iarray[96] = 0
-            rec = solver.solve(mm)
+            # on the resident matrix: values uploaded again without a rebuild would keep
+            # the plain solves below off the one-launch CG
+            rec = solver.solve_resident(mm.B, mm.X, mm.Iarray, mm.Rarray)
             assert rec["error"] == 0
         npairs = solver.learn_record(0)
         t1 = time.perf_counter()
@@ -1055,7 +1057,7 @@ def main():
         tag = "%dcube" % nx if nx == ny == nz else "%dx%dx%d" % (nx, ny, nz)
         cfg = config_dict(nx, ny, nz, m, args)
         cfg["solver"] = {"fp64": "plain FP64 CG + SSOR (drop-in)",
-                         "mixed": "FP64 CG + SSOR with BF16-stored factors (Iarray(42)=1)",
+                         "mixed": "FP64 CG + SSOR called with Iarray(42)=1: the one FP64 launch, as without",
                          "learned_fp64": "flexible CG, learned two-level preconditioner (SSOR two-grid cycle with "
                                          "the coarse space the network shapes), FP64 (Iarray(43)=1)",
                          "learned_mixed": "flexible CG, learned two-level preconditioner with BF16-stored SSOR and "
@@ -1064,7 +1066,7 @@ def main():
             "metric": METRIC, "value": dev_s, "unit": "s", "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": dev_s * 1e3, "higher_is_better": False,
             "scaling": "weak", "vs_baseline": None,
-            "dtype": "f64" if head in ("fp64", "learned_fp64") else "f64+bf16",
+            "dtype": "f64+bf16" if head.startswith(("learned_mixed", "twolevel")) else "f64",
             "data": "synthetic", "config": cfg,
             "variants": variants,
             "training": train,
