@@ -395,6 +395,8 @@ __device__ void team_solve_fused(const BatchArgs &a, int id, Team &t, CgState &s
       if (st.zero_rhs) a.x[3 * node + c] = 0.0;  // hecmw_solver.f90:32-37
       else a.px[3 * pos + c] = __ldcg(&a.x[3 * node + c]);
       a.v.zu[3 * size_t(pos) + c] = make_double2(0.0, 0.0);
+      a.v.p[3 * pos + c] = a.v.q[3 * pos + c] = a.v.h[3 * pos + c] = 0.0;
+      a.v.pl[3 * pos + c] = 0.0f;
     }
   }
   team_sync(t);

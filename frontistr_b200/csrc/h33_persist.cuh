@@ -36,7 +36,7 @@
 // a step is the latency of one slice per warp: a round of loads, 9 or 18 fused
 // multiply-adds per block, the lane sums, the 3x3 solve.  Measured per iteration against
 // the colour launches (us): 378 nodes 62 / 181, 19 thousand 110 / 305, 118 thousand
-// 179 / 372, 275 thousand 288 / 501, 1.03 million 716 / 1125.
+// 179 / 372, 275 thousand 288 / 501, 1.03 million 707 / 1125.
 // Measured and dropped: the blocks through shared-memory rings filled by bulk copies
 // (819 to 1000 us at 1.03 million nodes: 750 instructions a slice against 300, and a
 // ring of 12 KB a warp holds little more than the slice in work); the next slice's
@@ -261,6 +261,10 @@ __device__ __forceinline__ double ssor_sweep(const SsorVecs &a, const double *va
   const bool up = HALVES && (sub & (K / 2)) != 0;
   const int cc = HALVES ? sub & (K / 2 - 1) : sub, c0 = min(cc, 2);
   const size_t n = size_t(a.n);
+  // In the first iteration BETA is 0 and p, q, h and pl hold zeros.  Over the grid with 8 and
+  // 16 lanes not reading them then is 1 to 2 % of a solve the faster (less is in flight at
+  // once), in a cluster or a team and with 4 lanes reading them always is, by as much.
+  const bool fresh = first && K >= 8 && !CLUSTER;
   double dot = 0.0;
   int4 it = cur.next(), nx = cur.next();
   int col[U];
@@ -283,17 +287,17 @@ __device__ __forceinline__ double ssor_sweep(const SsorVecs &a, const double *va
         o0 = __ldcg(own + 3), o1 = __ldcg(own + 4), o2 = __ldcg(own + 5);
         f0 = __ldcg(a.g + i3 + c0);
         if (HALVES) {
-          if (!first) f1 = __ldcg((up ? a.q : a.h) + i3 + c0);
+          if (!fresh) f1 = __ldcg((up ? a.q : a.h) + i3 + c0);
           if (up) {
             f2 = __ldcg(own + c0);
-            if (!first) {
+            if (!fresh) {
               f3 = __ldcg(a.p + i3 + c0);
               fl = __ldcg(a.pl + i3 + c0);
             }
           }
         } else {
           f2 = __ldcg(own + c0);
-          if (!first) {
+          if (!fresh) {
             f1 = __ldcg(a.h + i3 + c0);
             f3 = __ldcg(a.p + i3 + c0);
             f4 = __ldcg(a.q + i3 + c0);
@@ -349,7 +353,7 @@ __device__ __forceinline__ double ssor_sweep(const SsorVecs &a, const double *va
           if (u < nx.y) col[u] = __ldg(cols + (nx.x + u) * 32 + lane);
       }
       // the direction here, beside the lane sums: after them its chain would be the step's
-      // tail (first: BETA, p and pl are zero)
+      // tail
       float rest = 0.0f;
       double pn = 0.0;
       if (MODE == 1) pn = next_direction(f2, beta, f3, fl, rest);
@@ -389,7 +393,7 @@ __device__ __forceinline__ double ssor_sweep(const SsorVecs &a, const double *va
           a.g[i] = cc == 0 ? e0 : cc == 1 ? e1 : e2;
         } else if (HALVES) {
           const double t = up ? f0 + lc : f0 - lc;  // g + L z, or g - L u
-          const double tn = first ? t : t + beta * f1;
+          const double tn = fresh ? t : t + beta * f1;
           (up ? a.q : a.h)[i] = tn;
           if (up) {
             a.p[i] = pn;
@@ -401,7 +405,7 @@ __device__ __forceinline__ double ssor_sweep(const SsorVecs &a, const double *va
         } else {
           const double mc = cc == 0 ? m[0] : cc == 1 ? m[1] : m[2];
           double qn = f0 + mc, hn = f0 - lc;
-          if (!first) {
+          if (!fresh) {
             qn = qn + beta * f4;
             hn = hn + beta * f1;
           }
@@ -551,13 +555,16 @@ __global__ void __launch_bounds__(32 * persist_warps<K>(), 1) cg_ssor_persist_ke
   const int gt = blockIdx.x * blockDim.x + tid, nt = gridDim.x * blockDim.x;
   GridWay way;
   persist_begin(a, sh);
-  // x in position order; z and u start at zero (padding blocks gather position 0)
+  // x in position order; z and u start at zero (padding blocks gather position 0), and what
+  // the first iteration reads of p, q, h and pl
   for (int i = gt; i < a.n; i += nt) {
     const int node = a.perm[i];
 #pragma unroll
     for (int c = 0; c < 3; c++) {
       a.px[3 * i + c] = a.x[3 * node + c];
       a.v.zu[3 * size_t(i) + c] = make_double2(0.0, 0.0);
+      a.v.p[3 * i + c] = a.v.q[3 * i + c] = a.v.h[3 * i + c] = 0.0;
+      a.v.pl[3 * i + c] = 0.0f;
     }
   }
   CgState &st = sh.st;
