@@ -8,7 +8,7 @@
 // handed a block's entries round by 19 shuffles, 26 blocks a row in the sweeps and 27 in
 // the product; here they pass through shared memory (5 vector loads a block) and L's serve
 // two products.  Measured per iteration with 16 load cases against the colour launches
-// (us): 378 nodes 152 / 204, 19 thousand 287 / 352 (8 warps a CTA), 118 thousand 695 / 783,
+// (us): 378 nodes 149 / 204, 19 thousand 287 / 352 (8 warps a CTA), 118 thousand 696 / 783,
 // but 275 thousand 1521 / 1477 (with the row's vectors still loaded one by one), where 105 MB
 // a vector stream through HBM and the launches' 24 warps an SM hide it better
 // (run_multi_chunk's rule).  Measured and dropped: 20 or 24

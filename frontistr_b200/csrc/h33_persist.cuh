@@ -35,8 +35,8 @@
 // runs as one cluster of 16 CTAs, whose hardware barrier takes 0.25 us.  What is left of
 // a step is the latency of one slice per warp: a round of loads, 9 or 18 fused
 // multiply-adds per block, the lane sums, the 3x3 solve.  Measured per iteration against
-// the colour launches (us): 378 nodes 62 / 181, 19 thousand 110 / 305, 118 thousand
-// 179 / 372, 275 thousand 288 / 501, 1.03 million 707 / 1125.
+// the colour launches (us): 378 nodes 62 / 181, 19 thousand 109 / 305, 118 thousand
+// 178 / 372, 275 thousand 285 / 501, 1.03 million 707 / 1125.
 // Measured and dropped: the blocks through shared-memory rings filled by bulk copies
 // (819 to 1000 us at 1.03 million nodes: 750 instructions a slice against 300, and a
 // ring of 12 KB a warp holds little more than the slice in work); the next slice's

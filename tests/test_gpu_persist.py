@@ -269,7 +269,7 @@ def test_attainable_accuracy_is_the_oracles(call, monkeypatch):
     left: no wider than hecmw_solve_CG's.  Geometric mean over 40 loads of the ratio of the
     two true residuals after 49 iterations; its standard error is 0.05.  The loops with a
     launch per colour give 0.89 to 0.99, the fused iteration gave 1.64 to 1.74 with the
-    rounding of p = z + BETA p left out of q and gives 0.94 to 1.08 with it.  The bound is
+    rounding of p = z + BETA p left out of q and gives 0.99 to 1.06 with it.  The bound is
     the middle of the two on a logarithmic scale, four standard errors from either."""
     m = graded_chain()
     m.set_iter(49)
